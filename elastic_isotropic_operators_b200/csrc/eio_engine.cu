@@ -21,6 +21,7 @@
 #include "eio_internal.h"
 #include "eio_kernels.cuh"
 #include "eio_pair.cuh"
+#include "eio_resident.cuh"
 #include "eio_sweep.cuh"
 #include "eio_tile.cuh"
 #include "eio_wave.cuh"
@@ -172,6 +173,9 @@ struct Engine {
     // kind 5 = two fine steps per launch (k_pair) with kind 3 for single steps
     int kind = 1, tz = 64, cw = 8, cpr = 8;
     bool tuned = false;
+    bool pinned = false;      // the kernel choice came from the caller: no resident loop
+    // resident time loop (eio_resident.cuh): shot table, step weights, edge slots, point tables
+    DBuf res_shot, res_step, res_x, res_map, res_first[2], res_pt[2];
     // tensor maps of the sweep kernel (valid for mtz/mcw)
     int mtz = -1, mcw = -1;
     CUtensorMap mwf_halo[10], mwf_int[10], mpar_halo[5], mpar_int[5];
@@ -386,7 +390,9 @@ void engine_destroy(Engine* e) {
     if (e->st2) cudaStreamSynchronize(e->st2);
     DBuf* all[] = {&e->dampz, &e->dampx, &e->inj_ts, &e->inj_ent, &e->inj_hts, &e->inj_hent, &e->ext_ts, &e->ext_ent,
                    &e->W, &e->err, &e->wsave,
-                   &e->Wq, &e->wscale, &e->wstage, &e->wpmax, &e->dampz_fs, &e->fsc, &e->dampx_w};
+                   &e->Wq, &e->wscale, &e->wstage, &e->wpmax, &e->dampz_fs, &e->fsc, &e->dampx_w,
+                   &e->res_shot, &e->res_step, &e->res_x, &e->res_map, &e->res_first[0],
+                   &e->res_first[1], &e->res_pt[0], &e->res_pt[1]};
     for (DBuf* b : all) b->release();
     for (int k = 0; k < 4; k++) {
         e->rint[k].slot.release(); e->rint[k].w.release(); e->rint[k].start.release(); e->rint[k].ent.release();
@@ -470,6 +476,13 @@ static void bucket(const std::vector<std::pair<int, PointEntry>>& tmp, int ntile
     for (auto& t : tmp) pl.ent[cur[t.first]++] = t.second;
 }
 
+static void check_point(const Engine* e, int cell) {
+    const int ix = cell / e->nz, iz = cell % e->nz;
+    if (cell < 0 || ix < FAT || ix >= e->nx - FAT || iz < FAT || iz >= e->nz - FAT)
+        throw Error(EIO_ERR_BOUNDS, "acquisition point " + std::to_string(cell) +
+                                        " lies outside the updated interior of the grid");
+}
+
 // Sort the points of the four position lists into per-tile buckets.
 static void build_points(const Engine* e, const int* const pos[4], const int npos[4], PointList& pl) {
     pl.pos = pos;
@@ -484,9 +497,7 @@ static void build_points(const Engine* e, const int* const pos[4], const int npo
         for (int k = 0; k < npos[g]; k++) {
             const int cell = pos[g][k];
             const int ix = cell / e->nz, iz = cell % e->nz;
-            if (cell < 0 || ix < FAT || ix >= e->nx - FAT || iz < FAT || iz >= e->nz - FAT)
-                throw Error(EIO_ERR_BOUNDS, "acquisition point " + std::to_string(cell) +
-                                                " lies outside the updated interior of the grid");
+            check_point(e, cell);
             const int bz = (iz - FAT) / tg.tz, bx = (ix - FAT) / tg.tx;
             PointEntry pe;
             pe.key = (f << 16) | (((ix - FAT) % tg.tx) << 8) | ((iz - FAT) % tg.tz);
@@ -980,6 +991,13 @@ void engine_set_kernel(Engine* e, int kind, int tz, int cw, int cpr) {
     e->tuned = true;
 }
 
+void engine_pin_kernel(Engine* e) { e->pinned = true; }
+void engine_copy_choice(Engine* to, const Engine* from) {
+    to->kind = from->kind; to->tz = from->tz; to->cw = from->cw; to->cpr = from->cpr;
+    to->tuned = from->tuned;
+    to->pinned = from->pinned;
+}
+
 // Columns [ix0, ix0 + nxw) of the grid as the grid of the next propagations
 // (nxw = 0: the whole grid).  The window keeps the grid's taper table: its
 // first and last FAT columns are the frozen frame and the taper runs from its
@@ -1163,13 +1181,316 @@ struct FsScope {
     ~FsScope() { e->fs_active = false; }
 };
 
+// ---------------------------------------------------------------- resident time loop
+// How a grid is cut into rectangles, one per CTA, and what a thread owns.
+struct ResPlan {
+    int Pz = 0, Px = 0, CB = 0, threads = 0, serv = 0, mq = 0, mx = 0;   // threads: compute threads, serv: service threads
+    bool pub = false;       // one unit per compute thread, which publishes its own edges
+    double cost = 1e30;     // modelled cycles of a fine step
+    int ctas() const { return Pz * Px; }
+};
+
+// dynamic shared memory of a CTA: the 227 KB it can have less the kernel's static part
+constexpr size_t RES_SMEM = 232448 - 1024;
+// Cells of a launch (all its shots) up to which the resident loop is taken,
+// forward and adjoint (which moves the fields themselves through L2).  It is
+// bound by the exchange of edges, a per-step launch by its latency on small
+// grids and by shared memory on large ones.  Microseconds a fine step, resident
+// against k_step: 312 x 520 (162 k cells) 4.2 / 6.1 forward, 4.5 / 6.2 adjoint;
+// three shots of 312 x 424 (397 k) 6.3 / 12.2 forward, 11.7 / 11.5 adjoint;
+// 1000 x 536 (536 k) 10.3 / 11.0 forward.
+constexpr long long RES_CELLS[2] = {420000, 200000};
+
+// Every way to cut an nz x nx grid (smallest window nx_min) into at most `ctas`
+// rectangles that the kernel can run, cheapest first.  The cost model: a unit
+// of the largest rectangle takes its LDS/STS.128 (51 a column, 37 for each of
+// two: an eighth of a cycle per lane) and the issue of its 410 instructions a
+// column; a phase cannot be shorter than the exchange of edges.
+static std::vector<ResPlan> res_plans(int nz, int nx, int nx_min, int ctas) {
+    std::vector<ResPlan> out;
+    const int nq = (nz - 2 * FAT) / 4, nc = nx - 2 * FAT, nc_min = nx_min - 2 * FAT;
+    for (int CB = 1; CB <= 2; CB++)
+        for (int Pz = 1; Pz <= std::min(ctas, nq); Pz++) {
+            const int ng = nc / CB;
+            for (int Px = std::min(ctas / Pz, ng); Px >= 1; Px--) {
+                ResPlan p;
+                p.Pz = Pz; p.Px = Px; p.CB = CB;
+                p.mq = (nq + Pz - 1) / Pz;
+                p.mx = (ng + Px - 1) / Px * CB;
+                if (res_smem(p.mq, p.mx, 0, 0) > RES_SMEM) break;   // fewer CTAs are larger still
+                if (nc_min / CB / Px * CB < FAT) continue;          // an edge comes from one neighbour
+                p.serv = std::min(std::max((res_edge(p.mq, p.mx) + 31) / 32 * 32, 64), 224);
+                const int units = res_rows(p.mq) * (p.mx / CB), most = RES_THREADS - p.serv,
+                          rounds = (units + most - 1) / most;
+                p.threads = ((units + rounds - 1) / rounds + 31) / 32 * 32;
+                p.pub = rounds == 1;
+                const double u = (double)p.threads * rounds * CB;
+                const double work = u * ((CB == 1 ? 51 : 37) / 8.0 + 410.0 / 128.0);
+                const double chain = 1500.0 + 800.0 * CB * rounds + 0.5 * res_edge(p.mq, p.mx) / 4.0;
+                p.cost = std::max(work, chain) + 0.4 * std::min(work, chain);
+                out.push_back(p);
+                break;                                      // the most CTAs along x for this Pz
+            }
+        }
+    std::sort(out.begin(), out.end(), [](const ResPlan& a, const ResPlan& b) { return a.cost < b.cost; });
+    return out;
+}
+
+// Points of one shot per CTA and unit (ResPoint).  False: a cell holds two
+// points of a field (the per-step kernels add them up).
+struct ResPoints {
+    std::vector<short> map;
+    std::vector<int> first;
+    std::vector<ResPoint> pt;
+    int cap = 0;
+    int ld[5] = {0, 0, 0, 0, 0};
+    bool any = false;
+};
+static bool res_points(const Engine* e, const ResPlan& p, const int* const pos[4], const int npos[4], ResPoints& o) {
+    const int nq = (e->nz - 2 * FAT) / 4, ng = (e->nx - 2 * FAT) / p.CB, ctas = p.ctas();
+    auto part = [](int i, int n, int parts) {   // the part [k n / parts, (k + 1) n / parts) that holds i
+        int k = (int)(((long long)i * parts) / n);
+        while ((long long)(k + 1) * n / parts <= i) k++;
+        while ((long long)k * n / parts > i) k--;
+        return k;
+    };
+    std::vector<std::vector<ResPoint>> of(ctas);
+    const int rows = res_rows(p.mq), stride = rows * p.mx;
+    o.any = false;
+    o.cap = 0;
+    for (int f = 0; f < 5; f++) {
+        const int g = kFieldGrid[f];
+        o.ld[f] = npos[g];
+        for (int k = 0; k < npos[g]; k++) {
+            const int cell = pos[g][k], ix = cell / e->nz, iz = cell % e->nz;
+            check_point(e, cell);
+            const int qz = (iz - FAT) / 4, gx = (ix - FAT) / p.CB;
+            const int pz = part(qz, nq, p.Pz), px = part(gx, ng, p.Px);
+            const int q0 = (int)((long long)pz * nq / p.Pz);
+            const int g0 = (int)((long long)px * ng / p.Px);
+            const int cta = px * p.Pz + pz;
+            const int u = cta * stride + ((gx - g0) * rows + qz - q0) * p.CB + (ix - FAT) % p.CB;
+            if (!o.any) {
+                o.any = true;
+                o.map.assign((size_t)ctas * stride, (short)-1);
+            }
+            if (o.map[u] < 0) {
+                if (of[cta].size() >= 32767) return false;
+                o.map[u] = (short)of[cta].size();
+                ResPoint r;
+                r.q = qz - q0;
+                r.x = ix - FAT - g0 * p.CB;
+                r.pad[0] = r.pad[1] = 0;
+                for (int a = 0; a < 5; a++)
+                    for (int j = 0; j < 4; j++) r.col[a][j] = -1;
+                of[cta].push_back(r);
+            }
+            int& col = of[cta][o.map[u]].col[f][(iz - FAT) % 4];
+            if (col >= 0) return false;
+            col = k;
+        }
+    }
+    o.first.assign(ctas + 1, 0);
+    o.pt.clear();
+    for (int c = 0; c < ctas; c++) {
+        o.pt.insert(o.pt.end(), of[c].begin(), of[c].end());
+        o.first[c + 1] = (int)o.pt.size();
+        o.cap = std::max(o.cap, (int)of[c].size());
+    }
+    return true;
+}
+
+// what a caller must leave alone for the resident loop to run: a pinned kernel
+// (eio_ctx_set_kernel), captured graphs and the free surface keep their launches
+static bool res_allowed(const Engine* e) { return !e->pinned && !e->use_graphs && !e->fs_active && !e->fs; }
+
+bool engine_resident(const Engine* e, int nx, int shots) {
+    return res_allowed(e) && (long long)e->nz * nx * shots <= RES_CELLS[1] && !res_plans(e->nz, nx, nx, e->nsm).empty();
+}
+
+// Cooperative launches of one device go one after another, whatever stream,
+// lane or context they come from: each waits for the one before.
+struct ResTurn {
+    std::mutex m;
+    cudaEvent_t last = nullptr;
+};
+static ResTurn& res_turn(int device) {
+    static ResTurn turns[64];
+    return turns[device & 63];
+}
+
+// One nonlinear propagation of nb shots (engines es, all of the first one's
+// device, grid height and time axis; each with its own window) as one launch.
+struct Resident {
+    Engine* const* es;
+    int nb;
+    ResPlan p;
+    std::vector<ResPoints> inj, ext;
+    std::vector<ResShot> sh;
+    std::vector<ResStep> steps;
+    int inj_cap = 0, ext_cap = 0;
+
+    Resident(Engine* const* engines, int n) : es(engines), nb(n), inj(n), ext(n), sh(n) {}
+
+    // The cheapest plan with all shots side by side whose point buffers fit
+    // too; false: no such plan, or not the better way.  g: acquisition per
+    // shot; the adjoint injects at the receivers.
+    bool plan(const ShotGeom* g, int adj) {
+        Engine* e0 = es[0];
+        int nx = 0, nx_min = 1 << 30;
+        long long cells = 0;
+        for (int i = 0; i < nb; i++) {
+            if (!res_allowed(es[i])) return false;
+            nx = std::max(nx, es[i]->nx);
+            nx_min = std::min(nx_min, es[i]->nx);
+            cells += es[i]->n;
+        }
+        if (cells > RES_CELLS[adj] || e0->nsm < nb) return false;
+        int tried = 0;
+        for (const ResPlan& c : res_plans(e0->nz, nx, nx_min, e0->nsm / nb)) {
+            if (tried++ == 6) break;
+            p = c;
+            inj_cap = ext_cap = 0;
+            for (int i = 0; i < nb; i++) {
+                if (!res_points(es[i], p, adj ? g[i].recPos : g[i].srcPos, adj ? g[i].nRec : g[i].nSrc, inj[i]) ||
+                    !res_points(es[i], p, adj ? g[i].srcPos : g[i].recPos, adj ? g[i].nSrc : g[i].nRec, ext[i]))
+                    return false;
+                inj_cap = std::max(inj_cap, inj[i].cap);
+                ext_cap = std::max(ext_cap, ext[i].cap);
+            }
+            if (res_smem(p.mq, p.mx, inj_cap, ext_cap) <= RES_SMEM) return true;
+        }
+        return false;
+    }
+
+    // edge slots of one shot, in uint4
+    size_t slots() const { return (size_t)4 * 2 * res_edge(p.mq, p.mx) * p.ctas(); }
+
+    // tables of every shot on its engine's stream (its signal buffers are set up);
+    // the first engine's stream is to wait for the others before run()
+    void prepare() {
+        Engine* e0 = es[0];
+        e0->res_x.ensure(sizeof(uint4) * slots() * nb);
+        for (int i = 0; i < nb; i++) {
+            Engine* e = es[i];
+            ResShot& s = sh[i];
+            memset(&s, 0, sizeof(s));
+            for (int f = 0; f < 5; f++) {
+                s.lev[0][f] = e->wf[f].f();
+                s.lev[1][f] = e->wf[5 + f].f();
+                s.par[f] = mpar(e0, f) + (long long)e->win_ix0 * e->nz;
+                s.inj_sig[f] = e->sig_in[f].f(); s.inj_ld[f] = inj[i].ld[f];
+                s.ext_sig[f] = e->sig_out[f].f(); s.ext_ld[f] = ext[i].ld[f];
+            }
+            s.dampz = e->dampz.f();
+            s.dampx = e->windowed ? e->dampx_w.f() : e->dampx.f();
+            s.nz = e->nz; s.nx = e->nx; s.Pz = p.Pz; s.Px = p.Px;
+            s.xbuf = static_cast<uint4*>(e0->res_x.p) + slots() * i;
+            for (int k = 0; k < 2; k++) {
+                const ResPoints& r = k ? ext[i] : inj[i];
+                if (!r.any) continue;
+                if (k == 0) upload(e->res_map, r.map.data(), sizeof(short) * r.map.size(), e->st);
+                upload(e->res_first[k], r.first.data(), sizeof(int) * r.first.size(), e->st);
+                upload(e->res_pt[k], r.pt.data(), sizeof(ResPoint) * r.pt.size(), e->st);
+            }
+            if (inj[i].any) {
+                s.inj_map = static_cast<const short*>(e->res_map.p);
+                s.inj_first = static_cast<const int*>(e->res_first[0].p);
+                s.inj_pt = static_cast<const ResPoint*>(e->res_pt[0].p);
+            }
+            if (ext[i].any) {
+                s.ext_first = static_cast<const int*>(e->res_first[1].p);
+                s.ext_pt = static_cast<const ResPoint*>(e->res_pt[1].p);
+            }
+        }
+    }
+
+    // every fine step, on the first engine's stream.  The adjoint's wavefield
+    // levels must be zero; this object's tables are read until the stream is done.
+    void run(int adj) {
+        Engine* e = es[0];
+        const float* F = e->filt.data();
+        const int h = e->h, S = e->S;
+        steps.clear();
+        steps.reserve((size_t)(e->nts - 1) * S);
+        for (int k = 0; k < (e->nts - 1) * S; k++) {
+            // engine_nl's order and weights
+            const int its = adj ? e->nts - 2 - k / S : k / S, it2 = adj ? S - 1 - k % S : k % S + 1;
+            const int ki = adj ? it2 + 1 : it2 - 1;
+            ResStep r;
+            r.inj_t = its; r.iw0 = F[ki]; r.iw1 = F[h + ki];
+            r.ext_t = its; r.ew0 = F[it2]; r.ew1 = F[h + it2];
+            r.ext_op = k == 0 ? RES_LOAD : k % S ? 0 : adj ? RES_DOWN : RES_UP;
+            r.pad = 0;
+            steps.push_back(r);
+        }
+        steps.back().ext_op |= RES_STORE;
+        upload(e->res_shot, sh.data(), sizeof(ResShot) * nb, e->st);
+        upload(e->res_step, steps.data(), sizeof(ResStep) * steps.size(), e->st);
+        EIO_CUDA(cudaMemsetAsync(e->res_x.p, 0, sizeof(uint4) * slots() * nb, e->st));   // no stale step matches
+        ResArgs a;
+        memset(&a, 0, sizeof(a));
+        a.shot = static_cast<const ResShot*>(e->res_shot.p);
+        a.step = static_cast<const ResStep*>(e->res_step.p);
+        a.nsteps = (int)steps.size();
+        a.nserv = p.serv;
+        a.pub = p.pub ? 1 : 0;
+        a.per_shot = p.ctas();
+        a.mq = p.mq; a.mx = p.mx;
+        a.map_stride = res_rows(p.mq) * p.mx;
+        a.inj_cap = inj_cap; a.ext_cap = ext_cap;
+        for (int k = 0; k < 4; k++) { a.cz[k] = e->zc[k]; a.cx[k] = e->xc[k]; }
+        a.err = static_cast<int*>(e->err.p);
+        a.wait_limit = e->wait_limit;
+        const void* fn = adj ? (p.CB == 1 ? (const void*)k_resident<1, 1> : (const void*)k_resident<1, 2>)
+                             : (p.CB == 1 ? (const void*)k_resident<0, 1> : (const void*)k_resident<0, 2>);
+        EIO_CUDA(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)RES_SMEM));
+        void* args[] = {&a};
+        {
+            ResTurn& t = res_turn(e->device);
+            std::lock_guard<std::mutex> lock(t.m);
+            if (!t.last) EIO_CUDA(cudaEventCreateWithFlags(&t.last, cudaEventDisableTiming));
+            else EIO_CUDA(cudaStreamWaitEvent(e->st, t.last, 0));
+            stats_mark(e);
+            EIO_CUDA(cudaLaunchCooperativeKernel(fn, dim3(nb * p.ctas()), dim3(p.threads + p.serv), args,
+                                                 res_smem(p.mq, p.mx, inj_cap, ext_cap), e->st));
+            stats_mark(e);
+            EIO_CUDA(cudaEventRecord(t.last, e->st));
+        }
+        // the counters keep counting fine steps: a launch of k steps is k step launches, all of them timed
+        e->launches++;
+        e->step_launches += a.nsteps;
+        if (e->stats) e->sampled += a.nsteps;
+        for (int i = 0; i < nb; i++) e->step_cells += (long long)(es[i]->nz - 2 * FAT) * (es[i]->nx - 2 * FAT) * a.nsteps;
+    }
+};
+
 void engine_nl(Engine* e, int adj, float* const model[5], float* const data[5], const ShotGeom& g, float* wfld) {
     EIO_CUDA(cudaSetDevice(e->device));
     if (wfld && e->windowed) throw Error(EIO_ERR_UNSUPPORTED, "saved wavefields cover the whole grid: no shot windows");
-    if (!e->tuned) engine_autotune(e);
     FsScope fs_scope(e);
-    err_reset(e);
     PointList src, rec;
+    if (!wfld && res_allowed(e)) {
+        build_points(e, g.srcPos, g.nSrc, src);
+        build_points(e, g.recPos, g.nRec, rec);
+        Resident r(&e, 1);
+        if (r.plan(&g, adj)) {
+            err_reset(e);
+            if (adj) zero_wavefields(e);
+            stage_in(e, adj ? data : model, adj ? rec.ld : src.ld, e->nts, e->sig_in);
+            zero_out(e, adj ? src.ld : rec.ld, e->nts, e->sig_out);
+            r.prepare();
+            r.run(adj);
+            check_launch();
+            stage_out(e, adj ? src.ld : rec.ld, e->nts, e->sig_out, adj ? model : data);
+            EIO_CUDA(cudaStreamSynchronize(e->st));
+            stats_flush(e);
+            err_check(e);
+            return;
+        }
+    }
+    if (!e->tuned) engine_autotune(e);
+    err_reset(e);
     build_points(e, g.srcPos, g.nSrc, src);
     build_points(e, g.recPos, g.nRec, rec);
     StepArgs a = base_args(e);
@@ -2042,7 +2363,12 @@ void engine_nl_shots_batch(Engine* const* es, int nb, int adj, float* const* mod
     if (nb < 1 || nb > STEP_BATCH) throw Error(EIO_ERR_ARG, "batch of 1 .. 8 shots");
     Engine* e0 = es[0];
     EIO_CUDA(cudaSetDevice(e0->device));
-    if (!e0->tuned) engine_autotune(e0);
+    Resident res(es, nb);
+    const bool resident = res.plan(g, adj);
+    if (!resident) {
+        if (!e0->tuned) engine_autotune(e0);
+        for (int i = 1; i < nb; i++) engine_copy_choice(es[i], e0);   // one tile geometry
+    }
     const int minb = (e0->kind == 3 || e0->kind == 5) ? 4 : 3;
     std::vector<PointList> src(nb), recp(nb);
     std::vector<Levels> lv;
@@ -2085,10 +2411,11 @@ void engine_nl_shots_batch(Engine* const* es, int nb, int adj, float* const* mod
             a.ext = upload_points(e, src[i], e->ext_ts, e->ext_ent, e->sig_out);
         }
         max_tiles = std::max(max_tiles, e->ntiles);
-        if (i > 0) {
-            EIO_CUDA(cudaEventRecord(e->ev_sync, e->st));
-            EIO_CUDA(cudaStreamWaitEvent(e0->st, e->ev_sync, 0));
-        }
+    }
+    if (resident) res.prepare();
+    for (int i = 1; i < nb; i++) {
+        EIO_CUDA(cudaEventRecord(es[i]->ev_sync, es[i]->st));
+        EIO_CUDA(cudaStreamWaitEvent(e0->st, es[i]->ev_sync, 0));
     }
     const float* F = e0->filt.data();
     const int h = e0->h;
@@ -2115,7 +2442,9 @@ void engine_nl_shots_batch(Engine* const* es, int nb, int adj, float* const* mod
         }
         launch();
     };
-    if (!adj) {
+    if (resident) {
+        res.run(adj);
+    } else if (!adj) {
         for (int its = 0; its < e0->nts - 1; its++)
             for (int it2 = 1; it2 < e0->S + 1; it2++) step(its, it2);
     } else {

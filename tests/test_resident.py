@@ -1,0 +1,146 @@
+"""The resident time loop of the nonlinear operators (small grids, whole
+propagation in one cooperative launch) against the per-step launches.
+
+A pinned kernel (eio_ctx_set_kernel) keeps the per-step launches, so each case
+runs once by default and once pinned to the tile kernel; both do the same
+operations in the same order, so their traces are the same bits.  Sizes: the
+smallest grid, one-row and ragged rectangles, both unit widths, both sides of
+the size rule, windows of different widths, several shots, sub > 1."""
+import ctypes
+import threading
+
+import numpy as np
+import pytest
+
+from elastic_isotropic_operators_b200 import _lib, prop, synthetic
+from helpers import Ctx, reg_inputs
+
+pytestmark = pytest.mark.gpu
+
+
+def _pair(w, windows=None):
+    ops = []
+    for pinned in (False, True):
+        src, rec = w.geometry()
+        op = prop.nonlinearPropElasticShotsGpu(w.elastic, w.par, *src, *rec)
+        if windows is not None:
+            op.setShotWindows(*windows)
+        if pinned:
+            _lib.check(op._L.eio_ctx_set_kernel(op.ctx, 0, 64, 16, 0))
+        ops.append(op)
+    return ops
+
+
+def _run(op, w, seed=3):
+    rng = np.random.default_rng(seed)
+    m, d = op.modelSpace(), op.dataSpace()
+    m.getNdArray()[...] = w.source_signal()[None]
+    op.forward(False, m, d)
+    a, b = op.modelSpace(), op.dataSpace()
+    b.getNdArray()[...] = rng.standard_normal(b.getNdArray().shape).astype(np.float32)
+    op.adjoint(False, a, b)
+    return d.getNdArray().copy(), a.getNdArray().copy()
+
+
+@pytest.mark.parametrize("nz,nx,nts,shots,sub", [
+    (40, 56, 40, 1, 1),      # smallest: rectangles of one float4 row or four columns
+    (72, 104, 61, 2, 1), (72, 104, 30, 3, 3), (104, 72, 40, 5, 2), (136, 264, 30, 8, 1),
+    (312, 520, 25, 1, 1),    # one unit per thread
+    (312, 424, 21, 3, 2),    # two columns per unit, several rounds (forward)
+    (328, 616, 21, 1, 1),    # adjoint just above its size rule
+    (56, 1256, 21, 1, 1), (1256, 56, 21, 2, 1)])
+def test_resident_equals_step_launches(nz, nx, nts, shots, sub):
+    w = synthetic.small(nz=nz, nx=nx, nts=nts, nshots=shots, nrec=min(20, (nx - 40) // 2), sub=sub, seed=nz + nx)
+    got, ref = (_run(op, w) for op in _pair(w))
+    for a, b in zip(got, ref):
+        assert np.abs(b).max() > 0
+        np.testing.assert_array_equal(a, b)
+
+
+def test_resident_windows():
+    w = synthetic.small(nz=72, nx=264, nts=60, nshots=2, nrec=20)
+    wins = ([0, 10], [8 + 16 * 16, 8 + 15 * 16])
+    got, ref = (_run(op, w) for op in _pair(w, wins))
+    for a, b in zip(got, ref):
+        np.testing.assert_array_equal(a, b)
+
+
+def test_resident_repeated_points_take_the_step_launches():
+    # a position given twice: its sources add up and both receivers record
+    w = synthetic.small(nts=40)
+    r = reg_inputs(w, "f", seed=4)
+    rep = lambda lists: [np.concatenate([p, p[:1]]) for p in lists]     # noqa: E731
+    sp, rp = rep(r["sp"]), rep(r["rp"])
+    model = [np.concatenate([m, m[:1]]) for m in r["model"]]
+    data = [np.concatenate([d, d[:1]]) for d in r["data"]]
+    out = []
+    for kind in (None, 0):
+        c = Ctx(w)
+        try:
+            if kind is not None:
+                c.set_kernel(kind)
+            out.append([c.nl(adj, model, data, sp, rp)[0 if adj else 1] for adj in (0, 1)])
+        finally:
+            c.close()
+    for a, b in zip(out[0], out[1]):
+        for x, y in zip(a, b):
+            np.testing.assert_allclose(x, y, rtol=0, atol=1e-6 * max(np.abs(y).max(), 1e-30))
+
+
+def test_resident_wait_timeout_reports_and_recovers():
+    w = synthetic.small(nts=60)
+    c = Ctx(w)
+    try:
+        r = reg_inputs(w, "f", seed=3)
+        for adj in (0, 1):
+            ref = c.nl(adj, r["model"], r["data"], r["sp"], r["rp"])[0 if adj else 1]
+            _lib.check(c.L.eio_ctx_set_wait_limit(c.h, 0))
+            with pytest.raises(prop.EioError) as ex:
+                c.nl(adj, r["model"], r["data"], r["sp"], r["rp"])
+            assert ex.value.code == -7
+            _lib.check(c.L.eio_ctx_set_wait_limit(c.h, -1))
+            got = c.nl(adj, r["model"], r["data"], r["sp"], r["rp"])[0 if adj else 1]
+            for a, b in zip(got, ref):
+                np.testing.assert_array_equal(a, b)
+    finally:
+        c.close()
+
+
+def test_resident_counts_fine_steps():
+    w = synthetic.small(nts=60, nshots=1)
+    op = _pair(w)[0]
+    m, d = op.modelSpace(), op.dataSpace()
+    m.getNdArray()[...] = w.source_signal()[None]
+    L, n, s, c = op._L, ctypes.c_longlong(), ctypes.c_longlong(), ctypes.c_longlong()
+    ms = ctypes.c_double()
+    _lib.check(L.eio_ctx_stats(op.ctx, 1, 1, None, None, None))
+    op.forward(False, m, d)
+    _lib.check(L.eio_ctx_stats(op.ctx, 1, 0, ctypes.byref(n), ctypes.byref(s), ctypes.byref(ms)))
+    _lib.check(L.eio_ctx_step_cells(op.ctx, ctypes.byref(c)))
+    assert s.value == w.fine_steps and n.value < 60 and ms.value > 0
+    assert c.value == w.fine_steps * w.cells
+
+
+def test_resident_contexts_on_threads():
+    # contexts of several host threads share the device; their cooperative launches take turns
+    w = synthetic.small(nz=104, nx=136, nts=80, nshots=2)
+    ref = _run(_pair(w)[0], w)
+    out, err = [None] * 4, []
+
+    def work(k):
+        try:
+            op = _pair(w)[0]
+            for _ in range(3):
+                out[k] = _run(op, w)
+        except Exception as e:     # noqa: BLE001
+            err.append(e)
+
+    th = [threading.Thread(target=work, args=(k,)) for k in range(4)]
+    for t in th:
+        t.start()
+    for t in th:
+        t.join()
+    assert not err, err
+    for o in out:
+        for a, b in zip(o, ref):
+            np.testing.assert_array_equal(a, b)
