@@ -1169,11 +1169,6 @@ static void save_wavefield(Engine* e, float* W, float* const p[5], int its, floa
     e->launches++;
 }
 
-static void fs_top(Engine* e, float* const c[5]) {
-    k_fs_top<<<(e->nx - 2 * FAT + 127) / 128, 128, 0, e->st>>>(c[0], c[1], c[3], c[4], e->nz, e->nx);
-    e->launches++;
-}
-
 // free-surface propagations run with the effective kind 0 while the guard lives
 struct FsScope {
     Engine* e;
@@ -1549,7 +1544,6 @@ void engine_nl(Engine* e, int adj, float* const model[5], float* const data[5], 
             L.set(a);
             weights(a, its, it2);
             if (!adj) {
-                if (e->fs_active) fs_top(e, L.c);
                 launch_step<0, EPI_NONE>(e, a, cur);
             } else {
                 launch_step<1, EPI_NONE>(e, a, cur);
