@@ -1031,6 +1031,228 @@ __global__ void __launch_bounds__(T_THREADS, CPS) k_conv_tma(const __grid_consta
         asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(Cf::TALLOC) : "memory");
 }
 
+// ---------------------------------------------------------------------------
+// k_conv_halo: the forward and data-gradient convolutions of wide images (128
+// pixels of a row per tile) with one copy of the input for all nine taps.
+// k_conv_tma fetches a box per tap, nine times the tile, in rows of 32 to 128
+// bytes, and TMA takes about eight cycles a row whatever its length (250 rows
+// per microsecond and SM here); the full-resolution layers of 16 to 96 channels
+// ran at that rate, tensor pipe and DRAM below 10 %.  Here a stage is the
+// tile's R image rows with their halo, (R + 2) x 130 pixels of every channel
+// block (box {cb, 130, R + 2}: 2 box rows per output pixel at R = 2 against 9),
+// and a tap is a whole number of pixel rows into it: the K-major operand of
+// output row r and tap (dy, dx) starts at pixel row (r + dy) 130 + dx, the
+// swizzle being a function of the shared-memory address.  The weights (9 cin x
+// cout) stay in shared memory for all tiles of the persistent CTA.  The sums
+// run over taps, channel blocks and K steps in k_conv_tma's order: same bits.
+// Measured, 16 images of 256 x 256 (B200, k_conv_tma with four CTAs per SM against
+// this): 16 -> 32 channels 93 / 40 us (15 at the HBM rate), 32 -> 32 126 / 60,
+// 32 -> 16 122 / 58, 32 -> 96 171 / 105, 64 -> 64 at 128 x 128 60 / 48; 96 -> 32,
+// whose three blocks leave one row a tile and one CTA an SM, 324 / 316.  Copies
+// by cp.async warps in place of TMA were slower (32 -> 32 88 us).
+constexpr int HALO_W = 128, HALO_P = HALO_W + 2;
+
+struct ConvHalo {
+    int C, cb, W, H, cpt;      // channels, channel block, image size, blocks per pixel
+    int tiles, stages;
+    int slab;                  // bytes of one channel block of a stage (a multiple of 1024)
+    int wbox;                  // weight boxes of 64 K
+    int N;                     // output channels
+    float* C32;
+    bf16* C16;
+    int relu;
+    long long wait;
+};
+
+template <int BN, int R>
+struct HCfg {
+    static constexpr int COLS = BN < 32 ? 32 : BN;
+    static constexpr int NEED = 2 * R * COLS;               // two buffers of R accumulators
+    static constexpr int TALLOC = NEED <= 64 ? 64 : NEED <= 128 ? 128 : NEED <= 256 ? 256 : 512;
+    static_assert(NEED <= 512, "accumulators fit the tensor memory");
+};
+
+template <int BN, int R>
+__global__ void __launch_bounds__(T_THREADS) k_conv_halo(const __grid_constant__ CUtensorMap ta,
+                                                        const __grid_constant__ CUtensorMap tb,
+                                                        const __grid_constant__ ConvHalo g)
+{
+    using Cf = HCfg<BN, R>;
+    extern __shared__ __align__(1024) unsigned char smem_raw[];
+    const unsigned raw = g_smem(smem_raw);
+    const unsigned w0 = raw + ((1024u - (raw & 1023u)) & 1023u);    // weights, then the stages
+    const unsigned s0 = w0 + (unsigned)(g.wbox * BN * 128);
+    const unsigned stage = (unsigned)(g.cpt * g.slab);
+    __shared__ __align__(8) unsigned long long bars[2 * 4 + 5];      // full[4], empty[4], tfull[2], tempty[2], weights
+    __shared__ unsigned tslot;
+    __shared__ int abort_flag, qprod, qmma;
+    volatile int* abort = &abort_flag;
+    auto full = [&](int s) { return g_smem(bars + s); };
+    auto empty = [&](int s) { return g_smem(bars + 4 + s); };
+    auto tfull = [&](int b) { return g_smem(bars + 8 + b); };
+    auto tempty = [&](int b) { return g_smem(bars + 10 + b); };
+    const unsigned wfull = g_smem(bars + 12);
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    const int S = g.stages;
+
+    if (tid == 0) {
+        for (int s = 0; s < 4; s++) {
+            asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(full(s)) : "memory");
+            asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(empty(s)) : "memory");
+        }
+        for (int b = 0; b < 2; b++) {
+            asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(tfull(b)) : "memory");
+            asm volatile("mbarrier.init.shared::cta.b64 [%0], 4;" ::"r"(tempty(b)) : "memory");
+        }
+        asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(wfull) : "memory");
+        abort_flag = 0;
+        qprod = 0;
+        qmma = 0;
+        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    }
+    if (warp == 1) {
+        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(g_smem(&tslot)),
+                     "r"(Cf::TALLOC)
+                     : "memory");
+        asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+    }
+    asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+    __syncthreads();
+    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+    const unsigned tmem = tslot;
+    // tile -> image, first row, first column; x fastest
+    const int tx = g.W / HALO_W, ty = g.H / R;
+    auto place = [&](int tile, int& n, int& y, int& x) {
+        x = tile % tx * HALO_W;
+        y = tile / tx % ty * R;
+        n = tile / (tx * ty);
+    };
+
+    if (warp == 0 && lane == 0) {
+        // ---- copies: the weights once, then a stage per tile
+        t_expect(wfull, (unsigned)(g.wbox * BN * 128));
+        for (int i = 0; i < g.wbox; i++) t_load2(w0 + (unsigned)(i * BN * 128), &tb, i * 64, 0, wfull);
+        int q = 0;
+        bool ok = true;
+        for (int tile = blockIdx.x; tile < g.tiles; tile += gridDim.x, q++) {
+            const int s = q % S;
+            if (!t_wait(empty(s), (unsigned)(((q / S) & 1) ^ 1), g.wait, abort)) {
+                ok = false;
+                break;
+            }
+            int n, y, x;
+            place(tile, n, y, x);
+            t_expect(full(s), (unsigned)(g.cpt * (R + 2) * HALO_P * g.cb * 2));
+            for (int c = 0; c < g.cpt; c++)
+                t_load4(s0 + (unsigned)s * stage + (unsigned)(c * g.slab), &ta, c * g.cb, x - 1, y - 1, n, full(s));
+        }
+        qprod = q;
+        if (!ok) *abort = 1;
+    } else if (warp == 1 && lane == 0) {
+        // ---- MMAs
+        const unsigned idesc = (1u << 4) | (1u << 7) | (1u << 10) | ((unsigned)(BN >> 3) << 17) |
+                               ((unsigned)(G_BM >> 4) << 24);
+        const int sw = 2 * g.cb;
+        int q = 0;
+        bool ok = t_wait(wfull, 0, g.wait, abort);
+        for (int tile = blockIdx.x; tile < g.tiles && ok; tile += gridDim.x, q++) {
+            const int b = q & 1, s = q % S;
+            if (!t_wait(tempty(b), (unsigned)(((q >> 1) & 1) ^ 1), g.wait, abort) ||
+                !t_wait(full(s), (unsigned)((q / S) & 1), g.wait, abort)) {
+                ok = false;
+                break;
+            }
+            asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+            const unsigned acc = tmem + (unsigned)(b * R * Cf::COLS);
+            int kk = 0;
+            for (int tap = 0; tap < 9; tap++)
+                for (int c = 0; c < g.cpt; c++) {
+                    const unsigned base = s0 + (unsigned)s * stage + (unsigned)(c * g.slab) +
+                                          (unsigned)((tap / 3 * HALO_P + tap % 3) * sw);
+                    for (int k = 0; k < g.cb / 16; k++, kk++) {
+                        const unsigned long long bd =
+                            t_desc(w0 + (unsigned)((kk >> 2) * BN * 128 + (kk & 3) * 32), 16, 1024, 128);
+#pragma unroll
+                        for (int r = 0; r < R; r++)
+                            t_mma(acc + (unsigned)(r * Cf::COLS),
+                                  t_desc(base + (unsigned)(r * HALO_P * sw + k * 32), 16, (unsigned)(8 * sw), sw), bd,
+                                  idesc, kk != 0);
+                    }
+                }
+            t_commit(empty(s));       // the stage is free once these MMAs have read it
+            t_commit(tfull(b));       // ... and the accumulators are complete
+        }
+        qmma = q;
+        if (!ok) *abort = 1;
+    } else if (warp >= 2) {
+        // ---- epilogue: warp w reads TMEM lanes 32 (w % 4) .. + 31, a pixel each
+        const int quarter = warp & 3;
+        int it = 0;
+        for (int tile = blockIdx.x; tile < g.tiles; tile += gridDim.x, it++) {
+            const int b = it & 1;
+            const bool seen = t_wait(tfull(b), (unsigned)((it >> 1) & 1), g.wait, abort);
+            if (!__all_sync(0xffffffffu, seen)) {
+                if (lane == 0) *abort = 1;
+                break;
+            }
+            asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+            int n, y, x;
+            place(tile, n, y, x);
+#pragma unroll 1
+            for (int rc = 0; rc < R * ((BN + 31) / 32); rc++) {
+                const int r = rc / ((BN + 31) / 32), c = rc % ((BN + 31) / 32) * 32;
+                const long long row = ((long long)n * g.H + y + r) * g.W + x + quarter * 32 + lane;
+                float v[32];
+                g_ld32(tmem + (unsigned)((b * R + r) * Cf::COLS + c) + ((unsigned)(quarter * 32) << 16), v);
+                const int nv = min(32, g.N - c);
+                if (nv <= 0) continue;
+                if (g.relu) {
+#pragma unroll
+                    for (int i = 0; i < 32; i++) v[i] = fmaxf(v[i], 0.f);
+                }
+                if (g.C32) {
+                    float* dst = g.C32 + row * g.N + c;
+#pragma unroll
+                    for (int i = 0; i < 32; i += 4)
+                        if (i < nv) *reinterpret_cast<float4*>(dst + i) = make_float4(v[i], v[i + 1], v[i + 2], v[i + 3]);
+                }
+                if (g.C16) {
+                    bf16* dst = g.C16 + row * g.N + c;
+#pragma unroll
+                    for (int i = 0; i < 32; i += 8)
+                        if (i < nv) {
+                            uint4 u;
+                            bf16* ub = reinterpret_cast<bf16*>(&u);
+#pragma unroll
+                            for (int e = 0; e < 8; e++) ub[e] = __float2bfloat16_rn(v[i + e]);
+                            *reinterpret_cast<uint4*>(dst + i) = u;
+                        }
+                }
+            }
+            asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+            __syncwarp();
+            if (lane == 0) t_arrive(tempty(b));
+        }
+    }
+    __syncthreads();
+    if (*abort && tid == 0) {
+        // drain: the weights, copies issued but never consumed, then the MMAs
+        const volatile int never = 0;
+        bool drained = t_wait(wfull, 0, G_DRAIN, &never);
+        for (int q = qmma; q < qprod; q++)
+            drained = t_wait(full(q % S), (unsigned)((q / S) & 1), G_DRAIN, &never) && drained;
+        if (qmma > 0) {
+            const int q = qmma - 1;
+            drained = t_wait(empty(q % S), (unsigned)((q / S) & 1), G_DRAIN, &never) && drained;
+        }
+        atomicMax(&g_gemm_err, drained ? 1 : 2);
+    }
+    asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+    __syncthreads();
+    if (warp == 1)
+        asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(Cf::TALLOC) : "memory");
+}
+
 int g_sms()
 {
     int dev = 0, n = 148;
@@ -1252,6 +1474,87 @@ int tma_wgrad_splits(long long M, long long P, long long* kchunk)
     return fit_splits(kt, (int)std::min<long long>(s, 4096), kchunk);
 }
 
+// ---- k_conv_halo: eligibility and launch
+struct HaloPlan {
+    int r, stages, ctas;       // output rows per tile, stages, CTAs per SM
+    size_t smem;
+};
+constexpr size_t H_SM = 227 * 1024;     // shared memory of an SM that CTAs can have
+
+// the deepest plan that fits: two rows per tile where the height allows, two
+// to four stages, as many CTAs per SM as tensor and shared memory hold
+bool halo_plan(int h, int w, int cin, int cout, HaloPlan* p)
+{
+    const int cb = chan_block(cin), bn = tma_bn(cout);
+    if (g_use_tma < 3 || !cb || w % HALO_W || cout % 16 || cout > bn || bn > 96) return false;
+    const int cpt = cin / cb;
+    const size_t wts = (size_t)((9LL * cin + 63) / 64) * bn * 128;
+    const int cols = std::max(bn, 32);
+    for (int r = h % 2 ? 1 : 2; r >= 1; r--) {
+        const size_t stage = (size_t)cpt * (((r + 2) * HALO_P * cb * 2 + 1023) / 1024 * 1024);
+        int talloc = 64;
+        while (talloc < 2 * r * cols) talloc *= 2;
+        for (int ctas = std::min(4, 512 / talloc); ctas >= 1; ctas--) {
+            const size_t most = H_SM / ctas - 2048;     // less the static part and the reserve
+            const long long st = ((long long)most - 1024 - (long long)wts) / (long long)stage;
+            if (st < 2 || (st < 3 && ctas > 2)) continue;
+            p->r = r;
+            p->ctas = ctas;
+            p->stages = (int)std::min<long long>(st, 4);
+            p->smem = most;
+            return true;
+        }
+    }
+    return false;
+}
+
+template <int BN, int R>
+void launch_halo(const CUtensorMap& ta, const CUtensorMap& tb, const ConvHalo& g, const HaloPlan& p, cudaStream_t st)
+{
+    GCUDA(cudaFuncSetAttribute(k_conv_halo<BN, R>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)p.smem));
+    const int grid = std::min(g.tiles, p.ctas * g_sms());
+    k_conv_halo<BN, R><<<(unsigned)grid, T_THREADS, p.smem, st>>>(ta, tb, g);
+    GCUDA(cudaGetLastError());
+}
+
+void conv_halo(int n, int h, int w, int cin, int cout, const void* x, const void* wt, float* y32, void* y16, int relu,
+               const HaloPlan& p, cudaStream_t st)
+{
+    const int bn = tma_bn(cout);
+    ConvHalo g{};
+    g.C = cin; g.cb = chan_block(cin); g.W = w; g.H = h; g.cpt = cin / g.cb;
+    const long long tiles = (long long)n * (h / p.r) * (w / HALO_W);
+    if (tiles > (1LL << 30)) throw Error(EIO_ERR_ARG, "conv3x3: too many tiles");
+    g.tiles = (int)tiles;
+    g.stages = p.stages;
+    g.slab = ((p.r + 2) * HALO_P * g.cb * 2 + 1023) / 1024 * 1024;
+    g.wbox = (int)((9LL * cin + 63) / 64);
+    g.N = cout;
+    g.C32 = y32;
+    g.C16 = static_cast<bf16*>(y16);
+    g.relu = relu;
+    g.wait = g_gemm_wait;
+    CUtensorMap ta, tb;
+    const cuuint64_t da[4] = {(cuuint64_t)cin, (cuuint64_t)w, (cuuint64_t)h, (cuuint64_t)n};
+    const cuuint64_t sa[3] = {(cuuint64_t)cin * 2, (cuuint64_t)w * cin * 2, (cuuint64_t)h * w * cin * 2};
+    const cuuint32_t ba[4] = {(cuuint32_t)g.cb, (cuuint32_t)HALO_P, (cuuint32_t)(p.r + 2), 1};
+    tma_map(&ta, x, 4, da, sa, ba, 2 * g.cb);
+    const cuuint64_t db[2] = {(cuuint64_t)(9LL * cin), (cuuint64_t)cout};
+    const cuuint64_t sb[1] = {(cuuint64_t)(9LL * cin * 2)};
+    const cuuint32_t bb[2] = {64, (cuuint32_t)bn};
+    tma_map(&tb, wt, 2, db, sb, bb, 128);
+    switch (bn * 2 + p.r - 1) {
+        case 16 * 2: launch_halo<16, 1>(ta, tb, g, p, st); break;
+        case 16 * 2 + 1: launch_halo<16, 2>(ta, tb, g, p, st); break;
+        case 32 * 2: launch_halo<32, 1>(ta, tb, g, p, st); break;
+        case 32 * 2 + 1: launch_halo<32, 2>(ta, tb, g, p, st); break;
+        case 64 * 2: launch_halo<64, 1>(ta, tb, g, p, st); break;
+        case 64 * 2 + 1: launch_halo<64, 2>(ta, tb, g, p, st); break;
+        case 96 * 2: launch_halo<96, 1>(ta, tb, g, p, st); break;
+        default: launch_halo<96, 2>(ta, tb, g, p, st); break;
+    }
+}
+
 unsigned chunks(long long values, const char* what)
 {
     if (values % 8) throw Error(EIO_ERR_ARG, std::string(what) + ": value counts must be multiples of 8");
@@ -1333,6 +1636,11 @@ void unet_conv3x3(int n, int h, int w, int cin, int cout, const void* x, const v
     if (!y32 && !y16) throw Error(EIO_ERR_ARG, "conv3x3: no output");
     check16opt(y32, "FP32 output");
     check16opt(y16, "BF16 output");
+    HaloPlan hp;
+    if (halo_plan(h, w, cin, cout, &hp)) {
+        conv_halo(n, h, w, cin, cout, x, wt, y32, y16, relu, hp, static_cast<cudaStream_t>(stream));
+        return;
+    }
     if (tma_conv_ok(h, w, cin)) {
         int bw, bh;
         rect_box(h, w, 128, &bw, &bh);
