@@ -122,6 +122,7 @@ _SIGS = {
     "eio_unet_flip": (I, [I, I, P, P, P]),
     "eio_unet_resample": (I, [I, I, I, I, I, P, P, I, P]),
     "eio_unet_concat": (I, [I, ctypes.c_longlong, I, I, P, I, P, I, P, P]),
+    "eio_unet_up_concat": (I, [I, I, I, I, I, I, P, P, P, P]),
     "eio_unet_relu_adj": (I, [ctypes.c_longlong, P, P, P, I, P]),
     "eio_ctx_pair_stats": (I, [P, ctypes.POINTER(ctypes.c_longlong), ctypes.POINTER(ctypes.c_double)]),
     "eio_nl_fwd_reg": (I, [P, P, P, P, IP, P, IP]),

@@ -610,6 +610,42 @@ __global__ void __launch_bounds__(MSE_THREADS) k_mse(const float* __restrict__ y
     }
 }
 
+// The same, 8 channels of a pixel per thread, for channel counts that are multiples of 8: 32-bit index
+// arithmetic, 16-byte stores, and no read of the channels without a target.  Bound by memory (C = 16, nc = 3:
+// 32 B of y, 12 of the target, 32 of dz a pixel; 1 M pixels 86 -> 22 us).
+__global__ void __launch_bounds__(MSE_THREADS) k_mse8(const float* __restrict__ y, const float* __restrict__ tgt,
+                                                      unsigned units, unsigned c8, int nc, float scale,
+                                                      bf16* __restrict__ dz, double* __restrict__ part)
+{
+    double acc = 0.0;
+    for (unsigned i = blockIdx.x * MSE_THREADS + threadIdx.x; i < units; i += gridDim.x * MSE_THREADS) {
+        const unsigned p = i / c8;
+        const int c0 = (int)(i - p * c8) * 8, n = min(nc - c0, 8);
+        uint4 u = make_uint4(0u, 0u, 0u, 0u);
+        bf16* const o = reinterpret_cast<bf16*>(&u);
+        const float* const ys = y + (long long)i * 8;
+        const float* const ts = tgt + (long long)p * nc + c0;
+#pragma unroll
+        for (int k = 0; k < 8; k++)
+            if (k < n) {
+                const float d = ys[k] - ts[k];
+                acc += (double)d * d;
+                o[k] = __float2bfloat16_rn(d * scale);
+            }
+        *reinterpret_cast<uint4*>(dz + (long long)i * 8) = u;
+    }
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) acc += __shfl_down_sync(0xffffffffu, acc, o);
+    __shared__ double ws[MSE_THREADS / 32];
+    if ((threadIdx.x & 31) == 0) ws[threadIdx.x >> 5] = acc;
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        double s = 0.0;
+        for (int k = 0; k < MSE_THREADS / 32; k++) s += ws[k];
+        part[blockIdx.x] = s;
+    }
+}
+
 // one warp: lane l sums part[l], part[l + 32], ... in order, then a fixed shuffle tree
 __global__ void k_sum_double(const double* __restrict__ part, int m, double scale, double* __restrict__ out)
 {
@@ -847,7 +883,12 @@ void cnn_mse(long long npix, int c, int nc, const float* y32, const float* targe
     if (!y32 || !target || !dz || !part || !loss) throw Error(EIO_ERR_ARG, "null loss buffer");
     auto st = static_cast<cudaStream_t>(stream);
     const double cnt = (double)npix * nc;
-    k_mse<<<nPart, MSE_THREADS, 0, st>>>(y32, target, npix, c, nc, (float)(1.0 / cnt), static_cast<bf16*>(dz), part);
+    // 16-byte stores need their alignment, 32-bit unit indices room for the grid's stride
+    if (c % 8 == 0 && reinterpret_cast<uintptr_t>(dz) % 16 == 0 && npix * (c / 8) < (1LL << 31))
+        k_mse8<<<nPart, MSE_THREADS, 0, st>>>(y32, target, (unsigned)(npix * (c / 8)), (unsigned)(c / 8), nc,
+                                              (float)(1.0 / cnt), static_cast<bf16*>(dz), part);
+    else
+        k_mse<<<nPart, MSE_THREADS, 0, st>>>(y32, target, npix, c, nc, (float)(1.0 / cnt), static_cast<bf16*>(dz), part);
     CCUDA(cudaGetLastError());
     k_sum_double<<<1, 32, 0, st>>>(part, nPart, 0.5 / cnt, loss);
     CCUDA(cudaGetLastError());

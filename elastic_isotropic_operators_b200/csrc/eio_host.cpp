@@ -1902,6 +1902,9 @@ EIO_API int eio_unet_concat(int adj, long long pixels, int ca, int cb, void* a, 
                             void* stream) {
     return guarded([&] { unet_concat(adj, pixels, ca, cb, a, addA, b, addB, z, stream); });
 }
+EIO_API int eio_unet_up_concat(int adj, int n, int h, int w, int ca, int cb, void* a, void* b, void* z, void* stream) {
+    return guarded([&] { unet_up_concat(adj, n, h, w, ca, cb, a, b, z, stream); });
+}
 EIO_API int eio_unet_relu_adj(long long n, const void* src, const void* mask, void* dst, int add, void* stream) {
     return guarded([&] { unet_relu_adj(n, src, mask, dst, add, stream); });
 }

@@ -182,5 +182,6 @@ void unet_flip(int cout, int cin, const void* w, void* wf, void* stream);
 void unet_resample(int op, int n, int h, int w, int c, const void* in, void* out, int add, void* stream);
 void unet_concat(int adj, long long pixels, int ca, int cb, void* a, int add_a, void* b, int add_b, void* z,
                  void* stream);
+void unet_up_concat(int adj, int n, int h, int w, int ca, int cb, void* a, void* b, void* z, void* stream);
 void unet_relu_adj(long long n, const void* src, const void* mask, void* dst, int add, void* stream);
 }  // namespace eio

@@ -274,9 +274,8 @@ class UNet:
         b = self.base
         L = [(n, h, w), (n, h // 2, w // 2), (n, h // 4, w // 4), (n, h // 8, w // 8)]
         spec = dict(e1a=(0, b), s1=(0, b), p1=(1, b), e2a=(1, 2 * b), s2=(1, 2 * b), p2=(2, 2 * b),
-                    e3a=(2, 4 * b), s3=(2, 4 * b), p3=(3, 4 * b), b=(3, 8 * b), u3=(2, 8 * b), c3=(2, 12 * b),
-                    d3=(2, 4 * b), u2=(1, 4 * b), c2=(1, 6 * b), d2=(1, 2 * b), u1=(0, 2 * b), c1=(0, 3 * b),
-                    d1=(0, b))
+                    e3a=(2, 4 * b), s3=(2, 4 * b), p3=(3, 4 * b), b=(3, 8 * b), c3=(2, 12 * b), d3=(2, 4 * b),
+                    c2=(1, 6 * b), d2=(1, 2 * b), c1=(0, 3 * b), d1=(0, b))
         t = lambda lv, c: torch.empty(L[lv] + (c,), dtype=bf, device=self.dev)
         self.a = {k: t(lv, c) for k, (lv, c) in spec.items()}     # activations
         self.g = {k: t(lv, c) for k, (lv, c) in spec.items()}     # their gradients
@@ -343,11 +342,10 @@ class UNet:
             nn, hh, ww = self.levels[lv]
             check(L.eio_unet_resample(0, nn, hh, ww, c, _p(src), _p(dst), 0, st))
 
-        def up_cat(src, lv, cu, skip, cs, up, cat):
+        def up_cat(src, lv, cu, skip, cs, cat):
             # cat = [up2(src), skip] at level lv - 1
             nn, hh, ww = self.levels[lv]
-            check(L.eio_unet_resample(2, nn, hh, ww, cu, _p(src), _p(up), 0, st))
-            check(L.eio_unet_concat(0, self._npix(lv - 1), cu, cs, _p(up), 0, _p(skip), 0, _p(cat), st))
+            check(L.eio_unet_up_concat(0, nn, hh, ww, cu, cs, _p(src), _p(skip), _p(cat), st))
 
         self._conv(0, x, 0, out16=a["e1a"])
         self._conv(1, a["e1a"], 0, out16=a["s1"])
@@ -359,11 +357,11 @@ class UNet:
         self._conv(5, a["e3a"], 2, out16=a["s3"])
         pool(a["s3"], 2, 4 * b, a["p3"])
         self._conv(6, a["p3"], 3, out16=a["b"])
-        up_cat(a["b"], 3, 8 * b, a["s3"], 4 * b, a["u3"], a["c3"])
+        up_cat(a["b"], 3, 8 * b, a["s3"], 4 * b, a["c3"])
         self._conv(7, a["c3"], 2, out16=a["d3"])
-        up_cat(a["d3"], 2, 4 * b, a["s2"], 2 * b, a["u2"], a["c2"])
+        up_cat(a["d3"], 2, 4 * b, a["s2"], 2 * b, a["c2"])
         self._conv(8, a["c2"], 1, out16=a["d2"])
-        up_cat(a["d2"], 1, 2 * b, a["s1"], b, a["u1"], a["c1"])
+        up_cat(a["d2"], 1, 2 * b, a["s1"], b, a["c1"])
         self._conv(9, a["c1"], 0, out16=a["d1"])
         self._conv(10, a["d1"], 0, out32=self.y32, relu=0)
         return self.y32
@@ -383,11 +381,10 @@ class UNet:
         check(L.eio_cnn_mse(n * h * w, _COUT, self.nout, _p(self.y32), _p(target), _p(g["y"]), _p(self._part),
                             _p(self._loss), st))
 
-        def split_up(cat_grad, lv, cu, cs, up_grad, skip_grad, src_grad):
+        def split_up(cat_grad, lv, cu, cs, skip_grad, src_grad):
             # [d up, d skip] = d cat (the skip's gradient overwritten); d src = up2^T (d up)
-            check(L.eio_unet_concat(1, self._npix(lv), cu, cs, _p(up_grad), 0, _p(skip_grad), 0, _p(cat_grad), st))
             nn, hh, ww = self.levels[lv + 1]
-            check(L.eio_unet_resample(3, nn, hh, ww, cu, _p(up_grad), _p(src_grad), 0, st))
+            check(L.eio_unet_up_concat(1, nn, hh, ww, cu, cs, _p(src_grad), _p(skip_grad), _p(cat_grad), st))
 
         def pool_back(pooled_grad, lv, c, skip_grad):
             # the skip's gradient += pool^T (d pooled)
@@ -396,11 +393,11 @@ class UNet:
 
         self._conv_back(10, a["d1"], 0, None, g["y"], g["d1"])
         self._conv_back(9, a["c1"], 0, a["d1"], g["d1"], g["c1"])
-        split_up(g["c1"], 0, 2 * b, b, g["u1"], g["s1"], g["d2"])
+        split_up(g["c1"], 0, 2 * b, b, g["s1"], g["d2"])
         self._conv_back(8, a["c2"], 1, a["d2"], g["d2"], g["c2"])
-        split_up(g["c2"], 1, 4 * b, 2 * b, g["u2"], g["s2"], g["d3"])
+        split_up(g["c2"], 1, 4 * b, 2 * b, g["s2"], g["d3"])
         self._conv_back(7, a["c3"], 2, a["d3"], g["d3"], g["c3"])
-        split_up(g["c3"], 2, 8 * b, 4 * b, g["u3"], g["s3"], g["b"])
+        split_up(g["c3"], 2, 8 * b, 4 * b, g["s3"], g["b"])
         self._conv_back(6, a["p3"], 3, a["b"], g["b"], g["p3"])
         pool_back(g["p3"], 2, 4 * b, g["s3"])
         self._conv_back(5, a["e3a"], 2, a["s3"], g["s3"], g["e3a"])

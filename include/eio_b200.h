@@ -544,6 +544,10 @@ int eio_unet_resample(int op, int n, int h, int w, int c, const void *in, void *
  * z[p][0:ca], b[p] (+)= z[p][ca:] (accumulating where addA / addB != 0) */
 int eio_unet_concat(int adj, long long pixels, int ca, int cb, void *a, int addA, void *b, int addB, void *z,
                     void *stream);
+/* adj = 0: z = [2x nearest upsampling of a, b] in one pass; a [n][h][w][ca], b and z
+ * [n][2h][2w][cb], [..][ca + cb]; adj = 1: a = the upsampling's adjoint of z[..][0:ca],
+ * b = z[..][ca:] (both overwritten) */
+int eio_unet_up_concat(int adj, int n, int h, int w, int ca, int cb, void *a, void *b, void *z, void *stream);
 /* dst (+)= src * (mask > 0) over n BF16 values, n a multiple of 8 (the ReLU
  * derivative) */
 int eio_unet_relu_adj(long long n, const void *src, const void *mask, void *dst, int add, void *stream);

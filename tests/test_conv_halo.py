@@ -71,3 +71,38 @@ def test_halo_convolution_wait_timeout_reports_and_recovers():
         _lib.check(L.eio_gemm_set_wait_limit(-1))
     e, got = conv()
     assert e == 0 and torch.equal(got, ref)
+
+
+@pytest.mark.parametrize("n,h,w,ca,cb", [(1, 1, 1, 8, 8), (2, 3, 5, 64, 32), (3, 8, 16, 256, 128), (1, 40, 24, 16, 48)])
+def test_up_concat_equals_its_two_passes(n, h, w, ca, cb):
+    torch = pytest.importorskip("torch")
+    L = _lib.lib()
+    bf = lambda *s: torch.randn(*s, device="cuda").to(torch.bfloat16)  # noqa: E731
+    a, b, z = bf(n, h, w, ca), bf(n, 2 * h, 2 * w, cb), bf(n, 2 * h, 2 * w, ca + cb)
+    up, z1, z2 = bf(n, 2 * h, 2 * w, ca), torch.empty_like(z), torch.empty_like(z)
+    _lib.check(L.eio_unet_resample(2, n, h, w, ca, _p(a), _p(up), 0, None))
+    _lib.check(L.eio_unet_concat(0, 4 * n * h * w, ca, cb, _p(up), 0, _p(b), 0, _p(z1), None))
+    _lib.check(L.eio_unet_up_concat(0, n, h, w, ca, cb, _p(a), _p(b), _p(z2), None))
+    assert torch.equal(z1, z2)
+    a1, b1, a2, b2 = (torch.empty_like(t) for t in (a, b, a, b))
+    _lib.check(L.eio_unet_concat(1, 4 * n * h * w, ca, cb, _p(up), 0, _p(b1), 0, _p(z), None))
+    _lib.check(L.eio_unet_resample(3, n, h, w, ca, _p(up), _p(a1), 0, None))
+    _lib.check(L.eio_unet_up_concat(1, n, h, w, ca, cb, _p(a2), _p(b2), _p(z), None))
+    assert torch.equal(a1, a2) and torch.equal(b1, b2)
+
+
+@pytest.mark.parametrize("npix,c,nc", [(1, 8, 1), (777, 16, 3), (5000, 24, 17), (300000, 16, 16), (1000, 12, 3)])
+def test_loss_and_its_derivative(npix, c, nc):
+    torch = pytest.importorskip("torch")
+    L = _lib.lib()
+    y, t = torch.randn(npix, c, device="cuda"), torch.randn(npix, nc, device="cuda")
+    dz = torch.full((npix, c), float("nan"), dtype=torch.bfloat16, device="cuda")
+    part = torch.zeros(1024, dtype=torch.float64, device="cuda")
+    loss = torch.zeros(1, dtype=torch.float64, device="cuda")
+    _lib.check(L.eio_cnn_mse(npix, c, nc, _p(y), _p(t), _p(dz), _p(part), _p(loss), None))
+    d = y[:, :nc] - t
+    want = torch.zeros_like(dz)
+    want[:, :nc] = (d * np.float32(1.0 / (npix * nc))).to(torch.bfloat16)
+    assert torch.equal(dz, want)
+    ref = 0.5 * d.double().square().mean().item()      # the same FP32 differences, summed in FP64
+    assert abs(loss.item() - ref) <= 1e-12 * ref
