@@ -106,3 +106,27 @@ def test_loss_and_its_derivative(npix, c, nc):
     assert torch.equal(dz, want)
     ref = 0.5 * d.double().square().mean().item()      # the same FP32 differences, summed in FP64
     assert abs(loss.item() - ref) <= 1e-12 * ref
+
+
+@pytest.mark.parametrize("n,h,w,cin,cout", [      # at least two tiles per SM, else the split GEMM runs
+    (300, 1, 128, 16, 16), (100, 5, 128, 16, 32), (5, 120, 128, 32, 32), (4, 50, 384, 32, 16), (3, 151, 256, 48, 32),
+    (2, 150, 128, 96, 32), (2, 302, 128, 64, 64), (2, 101, 256, 64, 16), (20, 32, 256, 32, 32), (1, 6, 256, 32, 32)])
+def test_halo_weight_gradient(n, h, w, cin, cout):
+    """Against FP64 products of the same BF16 values: FP32 sums of n h w terms, relative L2 <= 1e-5 (as the
+    other weight-gradient kernels); reproducible."""
+    torch = pytest.importorskip("torch")
+    L = _lib.lib()
+    rng = np.random.default_rng(h * w + cin)
+    bf = lambda *s: torch.as_tensor(rng.standard_normal(s).astype(np.float32), device="cuda").to(torch.bfloat16)  # noqa: E731
+    x, dz = bf(n, h, w, cin), bf(n, h, w, cout)
+    need = ctypes.c_longlong()
+    _lib.check(L.eio_unet_wgrad_scratch(n, h, w, cin, cout, ctypes.byref(need)))
+    scratch = torch.full((need.value,), float("nan"), device="cuda")
+    dw = [torch.full((cout, 9, cin), float("nan"), device="cuda") for _ in range(2)]
+    for d in dw:
+        _lib.check(L.eio_unet_conv3x3_wgrad(n, h, w, cin, cout, _p(x), _p(dz), _p(d), _p(scratch), need.value, None))
+    xp = torch.nn.functional.pad(x.double(), (0, 0, 1, 1, 1, 1))
+    ref = torch.stack([torch.einsum("nhwo,nhwi->oi", dz.double(), xp[:, i:i + h, j:j + w])
+                       for i in range(3) for j in range(3)], 1)
+    assert torch.equal(dw[0], dw[1])
+    assert ((dw[0].double() - ref).norm() / ref.norm()).item() < 1e-5
