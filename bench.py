@@ -760,7 +760,9 @@ def run_ours_nl(args, ws, rank, local):
                     "d2h_bytes_per_step": int(sum(4 * t.numel() for t in d_dev))},
             "roofline": {"bound": "hbm", "achieved": round(ach, 1), "peak": peak, "unit": "GB/s",
                          "frac": round(ach / peak, 4), "traffic": None, "peak_source": pk,
-                         "kernel": kernel_name(L, ctx), "avg_launch_us": round(avg * 1e3, 3),
+                         "kernel": "k_resident (every fine step in one launch; figures per fine step)"
+                         if st["launches"] < st["step_launches"] else kernel_name(L, ctx),
+                         "avg_launch_us": round(avg * 1e3, 3),
                          "algorithmic_bytes_per_launch": st["bytes_per_cell"] * cells},
             "cpu_baseline": cpu, "clocks": clk, "gpu_launches": st["launches"]}
 
