@@ -38,6 +38,7 @@
 #include <cuda_runtime.h>
 
 #include <algorithm>
+#include <atomic>
 #include <cstdint>
 #include <string>
 
@@ -1718,10 +1719,24 @@ bool halo_plan(int h, int w, int cin, int cout, HaloPlan* p)
     return false;
 }
 
+// A kernel's dynamic shared memory maximum, once per device and to the most that any plan asks for: the
+// attribute is the function's, so a call that set its own plan's size could shrink it between another
+// thread's call and launch.
+void halo_open(const void* kernel, std::atomic<bool> (&opened)[64])
+{
+    int dev = 0;
+    GCUDA(cudaGetDevice(&dev));
+    if (dev < 0 || dev >= 64) throw Error(EIO_ERR_ARG, "device index above 63");
+    if (opened[dev].load(std::memory_order_acquire)) return;
+    GCUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)(H_SM - 2048)));
+    opened[dev].store(true, std::memory_order_release);
+}
+
 template <int BN, int R>
 void launch_halo(const CUtensorMap& ta, const CUtensorMap& tb, const ConvHalo& g, const HaloPlan& p, cudaStream_t st)
 {
-    GCUDA(cudaFuncSetAttribute(k_conv_halo<BN, R>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)p.smem));
+    static std::atomic<bool> opened[64] = {};
+    halo_open((const void*)k_conv_halo<BN, R>, opened);
     const int grid = std::min(g.tiles, p.ctas * g_sms());
     k_conv_halo<BN, R><<<(unsigned)grid, T_THREADS, p.smem, st>>>(ta, tb, g);
     GCUDA(cudaGetLastError());
@@ -1803,7 +1818,8 @@ bool wgrad_plan(int n, int h, int w, int cin, int cout, WgradPlan* p)
 template <int BN, int R>
 void launch_wgrad(const CUtensorMap& ta, const CUtensorMap& tb, const WgradHalo& g, const WgradPlan& p, cudaStream_t st)
 {
-    GCUDA(cudaFuncSetAttribute(k_wgrad_halo<BN, R>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)p.smem));
+    static std::atomic<bool> opened[64] = {};
+    halo_open((const void*)k_wgrad_halo<BN, R>, opened);
     k_wgrad_halo<BN, R><<<(unsigned)p.grid, T_THREADS, p.smem, st>>>(ta, tb, g);
     GCUDA(cudaGetLastError());
 }

@@ -4,6 +4,7 @@ summed in the same order, so the same bits.  Odd heights take one row per tile,
 even ones two; one to three channel blocks; every tile width; FP32 and BF16
 outputs with and without ReLU."""
 import ctypes
+import threading
 
 import numpy as np
 import pytest
@@ -130,3 +131,54 @@ def test_halo_weight_gradient(n, h, w, cin, cout):
                        for i in range(3) for j in range(3)], 1)
     assert torch.equal(dw[0], dw[1])
     assert ((dw[0].double() - ref).norm() / ref.norm()).item() < 1e-5
+
+
+def test_halo_kernels_on_threads():
+    """Layers of different channel counts share a kernel and take different shared memory.  Host threads that
+    run them at once, each on its own stream: every launch is accepted and gives the bits of a serial run."""
+    torch = pytest.importorskip("torch")
+    L = _lib.lib()
+    n, h, w, cout = 300, 1, 128, 32
+    bf = lambda *s: torch.randn(*s, device="cuda").to(torch.bfloat16)  # noqa: E731
+    jobs = []
+    for cin in (16, 32, 64):
+        x, wt, dz = bf(n, h, w, cin), bf(cout, 9, cin), bf(n, h, w, cout)
+        need = ctypes.c_longlong()
+        _lib.check(L.eio_unet_wgrad_scratch(n, h, w, cin, cout, ctypes.byref(need)))
+        y, dw = torch.empty(n, h, w, cout, device="cuda"), torch.empty(cout, 9, cin, device="cuda")
+        scratch = torch.empty(need.value, device="cuda")
+
+        def conv(st, cin=cin, x=x, wt=wt, y=y):    # one image: the launches are what counts
+            _lib.check(L.eio_unet_conv3x3(1, h, w, cin, cout, _p(x), _p(wt), _p(y), None, 0, st))
+
+        def wgrad(st, cin=cin, x=x, dz=dz, dw=dw, scratch=scratch):
+            _lib.check(L.eio_unet_conv3x3_wgrad(n, h, w, cin, cout, _p(x), _p(dz), _p(dw), _p(scratch),
+                                                scratch.numel(), st))
+        jobs += [(conv, y[:1], 20000), (wgrad, dw, 3000)]
+    want = []
+    for f, o, _ in jobs:
+        f(None)
+        torch.cuda.synchronize()
+        want.append(o.clone())
+        o.fill_(float("nan"))
+    err = []
+
+    def work(f, passes):
+        torch.zeros(1, device="cuda")      # the device's context is this thread's too
+        st = torch.cuda.Stream()
+        try:
+            for _ in range(passes):
+                f(ctypes.c_void_p(st.cuda_stream))
+        except Exception as e:     # noqa: BLE001
+            err.append(e)
+        st.synchronize()
+
+    torch.cuda.synchronize()
+    th = [threading.Thread(target=work, args=(f, k)) for f, _, k in jobs]
+    for t in th:
+        t.start()
+    for t in th:
+        t.join()
+    assert not err, err
+    for (_, o, _), ref in zip(jobs, want):
+        assert torch.equal(o, ref)
