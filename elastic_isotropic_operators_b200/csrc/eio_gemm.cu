@@ -1321,9 +1321,14 @@ struct WgradHalo {
     int cbB;                   // channels of dz (= N)
     int tiles, stages, ngrp;   // ngrp: groups of 128 / cb vertical taps that cover three
     int slab;                  // bytes of one channel block of a stage
+    int dz;                    // offset of dz in a stage (wgrad_dz)
     float* part;               // [grid][9 C][N]
     long long wait;
 };
+
+// Bytes from a stage's start to its dz: the slabs, rounded up to the 1024 bytes after which the widest swizzle
+// pattern repeats.  A 16-channel slab of three rows is 13056 bytes, and dz at 64 channels must start on the pattern.
+constexpr int wgrad_dz(int cpt, int cb, int r) { return (cpt * (r + 2) * WG_P * cb * 2 + 1023) / 1024 * 1024; }
 
 template <int BN, int R>
 __global__ void __launch_bounds__(T_THREADS) k_wgrad_halo(const __grid_constant__ CUtensorMap ta,
@@ -1333,7 +1338,7 @@ __global__ void __launch_bounds__(T_THREADS) k_wgrad_halo(const __grid_constant_
     extern __shared__ __align__(1024) unsigned char smem_raw[];
     const unsigned raw = g_smem(smem_raw);
     const unsigned s0 = raw + ((1024u - (raw & 1023u)) & 1023u);
-    const unsigned stage = (unsigned)(g.cpt * g.slab + R * HALO_W * BN * 2);
+    const unsigned stage = (unsigned)(g.dz + R * HALO_W * BN * 2);
     __shared__ __align__(8) unsigned long long bars[2 * 4 + 1];      // full[4], empty[4], all accumulators complete
     __shared__ unsigned tslot;
     __shared__ int abort_flag, qprod, qmma;
@@ -1378,7 +1383,7 @@ __global__ void __launch_bounds__(T_THREADS) k_wgrad_halo(const __grid_constant_
             const unsigned at = s0 + (unsigned)s * stage;
             t_expect(full(s), (unsigned)(g.cpt * (R + 2) * WG_P * g.cb * 2 + R * HALO_W * BN * 2));
             for (int c = 0; c < g.cpt; c++) t_load4(at + (unsigned)(c * g.slab), &ta, c * g.cb, x - 1, y - 1, n, full(s));
-            t_load4(at + (unsigned)(g.cpt * g.slab), &tb, 0, x, y, n, full(s));
+            t_load4(at + (unsigned)g.dz, &tb, 0, x, y, n, full(s));
         }
         qprod = q;
         if (!ok) *abort = 1;
@@ -1399,7 +1404,7 @@ __global__ void __launch_bounds__(T_THREADS) k_wgrad_halo(const __grid_constant_
                 break;
             }
             asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-            const unsigned at = s0 + (unsigned)s * stage, bt = at + (unsigned)(g.cpt * g.slab);
+            const unsigned at = s0 + (unsigned)s * stage, bt = at + (unsigned)g.dz;
             for (int r = 0; r < R; r++)
                 for (int k = 0; k < HALO_W; k += 16) {
                     const unsigned long long bd = t_desc(bt + (unsigned)((r * HALO_W + k) * swB), (unsigned)(64 * swB),
@@ -1800,7 +1805,7 @@ bool wgrad_plan(int n, int h, int w, int cin, int cout, WgradPlan* p)
         // a CTA's one partial result pays off over several tiles; k_conv_tma splits small images finer
         const long long tiles = (long long)n * (h / r) * (w / HALO_W);
         if (tiles < 2LL * g_sms() || tiles > (1LL << 30)) continue;
-        const size_t stage = (size_t)cpt * (r + 2) * WG_P * cb * 2 + (size_t)r * HALO_W * cout * 2;
+        const size_t stage = (size_t)wgrad_dz(cpt, cb, r) + (size_t)r * HALO_W * cout * 2;
         for (int ctas = std::min(4, 512 / talloc); ctas >= 1; ctas--) {
             const size_t most = H_SM / ctas - 2048;
             const long long st = ((long long)most - 1024 - (long long)tail) / (long long)stage;
@@ -1834,6 +1839,7 @@ void wgrad_halo(int n, int h, int w, int cin, int cout, const void* x, const voi
     g.stages = p.stages;
     g.ngrp = p.ngrp;
     g.slab = (p.r + 2) * WG_P * g.cb * 2;
+    g.dz = wgrad_dz(g.cpt, g.cb, p.r);
     g.part = part;
     g.wait = g_gemm_wait;
     CUtensorMap ta, tb;

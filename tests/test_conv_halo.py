@@ -110,7 +110,7 @@ def test_loss_and_its_derivative(npix, c, nc):
 
 
 @pytest.mark.parametrize("n,h,w,cin,cout", [      # at least two tiles per SM, else the split GEMM runs
-    (300, 1, 128, 16, 16), (100, 5, 128, 16, 32), (5, 120, 128, 32, 32), (4, 50, 384, 32, 16), (3, 151, 256, 48, 32),
+    (300, 1, 128, 16, 16), (300, 1, 128, 16, 64), (60, 5, 128, 32, 64), (100, 5, 128, 16, 32), (5, 120, 128, 32, 32), (4, 50, 384, 32, 16), (3, 151, 256, 48, 32),
     (2, 150, 128, 96, 32), (2, 302, 128, 64, 64), (2, 101, 256, 64, 16), (20, 32, 256, 32, 32), (1, 6, 256, 32, 32)])
 def test_halo_weight_gradient(n, h, w, cin, cout):
     """Against FP64 products of the same BF16 values: FP32 sums of n h w terms, relative L2 <= 1e-5 (as the
