@@ -1576,9 +1576,18 @@ void tma_map(CUtensorMap* m, const void* base, int rank, const cuuint64_t* dims,
     const CUtensorMapSwizzle sw = swz == 128 ? CU_TENSOR_MAP_SWIZZLE_128B
                                   : swz == 64 ? CU_TENSOR_MAP_SWIZZLE_64B
                                               : CU_TENSOR_MAP_SWIZZLE_32B;
-    const CUresult r = tma_encoder()(m, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, (cuuint32_t)rank, const_cast<void*>(base),
-                                     dims, strides, box, es, CU_TENSOR_MAP_INTERLEAVE_NONE, sw,
-                                     CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+    auto encode = [&] {
+        return tma_encoder()(m, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, (cuuint32_t)rank, const_cast<void*>(base), dims,
+                             strides, box, es, CU_TENSOR_MAP_INTERLEAVE_NONE, sw, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
+                             CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+    };
+    CUresult r = encode();
+    if (r == CUDA_ERROR_INVALID_CONTEXT) {   // a host thread's first CUDA call: the encoder takes no device by itself
+        int dev = 0;
+        GCUDA(cudaGetDevice(&dev));
+        GCUDA(cudaSetDevice(dev));
+        r = encode();
+    }
     if (r != CUDA_SUCCESS) throw Error(EIO_ERR_CUDA, "cuTensorMapEncodeTiled failed (" + std::to_string((int)r) + ")");
 }
 

@@ -182,3 +182,23 @@ def test_halo_kernels_on_threads():
     assert not err, err
     for (_, o, _), ref in zip(jobs, want):
         assert torch.equal(o, ref)
+
+
+def test_convolution_as_a_threads_first_call():
+    torch = pytest.importorskip("torch")
+    L = _lib.lib()
+    x = torch.randn(1, 4, 128, 16, device="cuda").to(torch.bfloat16)
+    wt = torch.randn(16, 9, 16, device="cuda").to(torch.bfloat16)
+    y = [torch.empty(1, 4, 128, 16, device="cuda") for _ in range(2)]
+    rc = []
+
+    def conv(o):
+        rc.append(L.eio_unet_conv3x3(1, 4, 128, 16, 16, _p(x), _p(wt), _p(o), None, 0, None))
+
+    conv(y[0])
+    torch.cuda.synchronize()
+    th = threading.Thread(target=conv, args=(y[1],))
+    th.start()
+    th.join()
+    torch.cuda.synchronize()
+    assert rc == [0, 0] and torch.equal(y[0], y[1])
