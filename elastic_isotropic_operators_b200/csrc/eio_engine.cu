@@ -294,6 +294,29 @@ static void stats_mark(Engine* e, bool pair = false) {
     EIO_CUDA(cudaEventRecord(e->ev[e->ev_used++], e->st));
 }
 
+// Cooperative launches (the resident loop, the persistent shot groups) of one
+// device go one after another, whatever stream, lane or context they come from:
+// each waits for the one before.  Their CTAs wait for one another, so two of
+// them side by side must never each hold a part of the SMs.
+struct CoopTurn {
+    std::mutex m;
+    cudaEvent_t last = nullptr;
+};
+static CoopTurn& coop_turn(int device) {
+    static CoopTurn turns[64];
+    return turns[device & 63];
+}
+static void launch_cooperative(Engine* e, const void* fn, int grid, int block, void** args, size_t smem) {
+    CoopTurn& t = coop_turn(e->device);
+    std::lock_guard<std::mutex> lock(t.m);
+    if (!t.last) EIO_CUDA(cudaEventCreateWithFlags(&t.last, cudaEventDisableTiming));
+    else EIO_CUDA(cudaStreamWaitEvent(e->st, t.last, 0));
+    stats_mark(e);
+    EIO_CUDA(cudaLaunchCooperativeKernel(fn, dim3(grid), dim3(block), args, smem, e->st));
+    stats_mark(e);
+    EIO_CUDA(cudaEventRecord(t.last, e->st));
+}
+
 static void upload(DBuf& b, const void* h, size_t bytes, cudaStream_t st) {
     b.ensure(std::max<size_t>(bytes, 16));
     if (bytes) EIO_CUDA(cudaMemcpyAsync(b.p, h, bytes, cudaMemcpyHostToDevice, st));
@@ -1303,17 +1326,6 @@ bool engine_resident(const Engine* e, int nx, int shots) {
     return res_allowed(e) && (long long)e->nz * nx * shots <= RES_CELLS[1] && !res_plans(e->nz, nx, nx, e->nsm).empty();
 }
 
-// Cooperative launches of one device go one after another, whatever stream,
-// lane or context they come from: each waits for the one before.
-struct ResTurn {
-    std::mutex m;
-    cudaEvent_t last = nullptr;
-};
-static ResTurn& res_turn(int device) {
-    static ResTurn turns[64];
-    return turns[device & 63];
-}
-
 // One nonlinear propagation of nb shots (engines es, all of the first one's
 // device, grid height and time axis; each with its own window) as one launch.
 struct Resident {
@@ -1441,17 +1453,7 @@ struct Resident {
                              : (p.CB == 1 ? (const void*)k_resident<0, 1> : (const void*)k_resident<0, 2>);
         EIO_CUDA(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)RES_SMEM));
         void* args[] = {&a};
-        {
-            ResTurn& t = res_turn(e->device);
-            std::lock_guard<std::mutex> lock(t.m);
-            if (!t.last) EIO_CUDA(cudaEventCreateWithFlags(&t.last, cudaEventDisableTiming));
-            else EIO_CUDA(cudaStreamWaitEvent(e->st, t.last, 0));
-            stats_mark(e);
-            EIO_CUDA(cudaLaunchCooperativeKernel(fn, dim3(nb * p.ctas()), dim3(p.threads + p.serv), args,
-                                                 res_smem(p.mq, p.mx, inj_cap, ext_cap), e->st));
-            stats_mark(e);
-            EIO_CUDA(cudaEventRecord(t.last, e->st));
-        }
+        launch_cooperative(e, fn, nb * p.ctas(), p.threads + p.serv, args, res_smem(p.mq, p.mx, inj_cap, ext_cap));
         // the counters keep counting fine steps: a launch of k steps is k step launches, all of them timed
         e->launches++;
         e->step_launches += a.nsteps;
@@ -2599,15 +2601,10 @@ void ShotBatch::run(const ImagingArgs* ia, float* const* slots) {
     w.nb = nb;
     w.max_tiles = max_tiles;
     const int units = nb * max_tiles;
-    const bool timed = e0->stats;
-    if (timed) stats_mark(e0);
     void* args[] = {&w};
     const int g = std::min(units, wave_resident<DIR, EPI, MINB>(e0, wave_slot<DIR, EPI, MINB>()));
-    EIO_CUDA(cudaLaunchCooperativeKernel((const void*)k_wave<DIR, EPI, MINB>, g, NT, args, 0, e0->st));
-    if (timed) {
-        stats_mark(e0);
-        e0->sampled += nsteps;   // the event pair covers every step of the phase
-    }
+    launch_cooperative(e0, (const void*)k_wave<DIR, EPI, MINB>, g, NT, args, 0);
+    if (e0->stats) e0->sampled += nsteps;   // the event pair covers every step of the phase
     e0->launches++;
     e0->step_launches += nsteps;
     batch_count(e0, es, nb, nsteps);

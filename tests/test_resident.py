@@ -144,3 +144,45 @@ def test_resident_contexts_on_threads():
     for o in out:
         for a, b in zip(o, ref):
             np.testing.assert_array_equal(a, b)
+
+
+def test_resident_beside_the_persistent_born_groups():
+    # the other cooperative launch of the library, on another context and host thread
+    w = synthetic.small(nz=104, nx=136, nts=60, nshots=3)
+    src, rec = w.geometry()
+    nl = _pair(w)[0]
+    born = prop.BornElasticShotsGpu(w.elastic, w.par, [w.source_signal()], *src, *rec)
+    born.setBornBatch(3)
+    born.setLanes(3)
+    _lib.check(born._L.eio_ctx_set_kernel(born.ctx, 3, 64, 16, 0))
+    born.setPersistent(7)
+
+    def run_born():
+        m, d = born.modelSpace(), born.dataSpace()
+        m.getNdArray()[...] = w.extra["dmodel"]
+        born.forward(False, m, d)
+        a = born.modelSpace()
+        born.adjoint(False, a, d)
+        return d.getNdArray().copy(), a.getNdArray().copy()
+
+    jobs = [lambda: _run(nl, w), run_born]
+    ref = [f() for f in jobs]
+    out, err = [[], []], []
+
+    def work(k):
+        try:
+            for _ in range(5):
+                out[k].append(jobs[k]())
+        except Exception as e:     # noqa: BLE001
+            err.append(e)
+
+    th = [threading.Thread(target=work, args=(k,)) for k in range(2)]
+    for t in th:
+        t.start()
+    for t in th:
+        t.join()
+    assert not err, err
+    for k in range(2):
+        for o in out[k]:
+            for a, b in zip(o, ref[k]):
+                np.testing.assert_array_equal(a, b)
