@@ -1320,7 +1320,7 @@ static bool res_points(const Engine* e, const ResPlan& p, const int* const pos[4
 
 // what a caller must leave alone for the resident loop to run: a pinned kernel
 // (eio_ctx_set_kernel), captured graphs and the free surface keep their launches
-static bool res_allowed(const Engine* e) { return !e->pinned && !e->use_graphs && !e->fs_active && !e->fs; }
+static bool res_allowed(const Engine* e) { return !e->pinned && !e->use_graphs && !e->fs; }
 
 bool engine_resident(const Engine* e, int nx, int shots) {
     return res_allowed(e) && (long long)e->nz * nx * shots <= RES_CELLS[1] && !res_plans(e->nz, nx, nx, e->nsm).empty();
@@ -1465,7 +1465,6 @@ struct Resident {
 void engine_nl(Engine* e, int adj, float* const model[5], float* const data[5], const ShotGeom& g, float* wfld) {
     EIO_CUDA(cudaSetDevice(e->device));
     if (wfld && e->windowed) throw Error(EIO_ERR_UNSUPPORTED, "saved wavefields cover the whole grid: no shot windows");
-    FsScope fs_scope(e);
     PointList src, rec;
     if (!wfld && res_allowed(e)) {
         build_points(e, g.srcPos, g.nSrc, src);
@@ -1486,7 +1485,8 @@ void engine_nl(Engine* e, int adj, float* const model[5], float* const data[5], 
             return;
         }
     }
-    if (!e->tuned) engine_autotune(e);
+    if (!e->tuned) engine_autotune(e);   // the choice serves the Born operators too: timed without the free surface
+    FsScope fs_scope(e);
     err_reset(e);
     build_points(e, g.srcPos, g.nSrc, src);
     build_points(e, g.recPos, g.nRec, rec);
