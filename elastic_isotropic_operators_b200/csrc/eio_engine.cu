@@ -1322,10 +1322,6 @@ static bool res_points(const Engine* e, const ResPlan& p, const int* const pos[4
 // (eio_ctx_set_kernel), captured graphs and the free surface keep their launches
 static bool res_allowed(const Engine* e) { return !e->pinned && !e->use_graphs && !e->fs; }
 
-bool engine_resident(const Engine* e, int nx, int shots) {
-    return res_allowed(e) && (long long)e->nz * nx * shots <= RES_CELLS[1] && !res_plans(e->nz, nx, nx, e->nsm).empty();
-}
-
 // One nonlinear propagation of nb shots (engines es, all of the first one's
 // device, grid height and time axis; each with its own window) as one launch.
 struct Resident {

@@ -410,15 +410,17 @@ static float* lane_staging(eio_ctx* c, int k, size_t n) {
 static Engine* lane_engine(eio_ctx* c, int k) { return k == 0 ? c->eng : c->extra[k - 1]; }
 
 static size_t lane_bytes(const eio_ctx* c, bool born);
-static int widest(const eio_ctx* c);
 // Lanes for a call over nShots shots, each lane needing about lane_bytes of
 // device memory for the call: at most c->lanes and nShots, fewer when the free
 // memory would not hold what the lanes still have to allocate (a new lane all
 // of it; an existing one its Born history, which is allocated at first use).
-// New lanes take the first lane's kernel choice (tuned first), checkpoint
+// Every lane takes the first lane's kernel choice, new ones also its checkpoint
 // precision and graph setting.
-// born: the lanes run Born propagations.
-static int ensure_lanes(eio_ctx* c, int nShots, bool born, int want = 0) {
+// born: the lanes run Born propagations.  tune: the choice is made here, before
+// the lanes run side by side (a lane that timed the kernels among the others'
+// work could choose any); the lockstep nonlinear groups make it on one thread,
+// when they need it.
+static int ensure_lanes(eio_ctx* c, int nShots, bool born, bool tune, int want = 0) {
     const size_t lane_bytes = ::lane_bytes(c, born);
     int n = std::max(1, std::min(want > 0 ? want : c->lanes, nShots));
     const int have = 1 + (int)c->extra.size();
@@ -439,9 +441,7 @@ static int ensure_lanes(eio_ctx* c, int nShots, bool born, int want = 0) {
             n = std::min(n, have);
         }
     }
-    // one kernel choice for all lanes, made before they run; the resident loop needs none
-    const bool resident = !born && engine_resident(c->eng, widest(c), n);
-    if (n > 1 && !resident && !engine_is_tuned(c->eng)) engine_autotune(c->eng);
+    if (n > 1 && tune && !engine_is_tuned(c->eng)) engine_autotune(c->eng);
     for (Engine* e : c->extra) engine_copy_choice(e, c->eng);
     while ((int)c->extra.size() < n - 1) {
         Engine* e = engine_create(c->device, c->fd);
@@ -494,7 +494,7 @@ static void run_lanes(eio_ctx* c, int n, int nShots, F&& f) {
 static int born_batch_width(eio_ctx* c, int nShots) {
     const int want = std::min(std::min(c->born_batch, c->lanes), (int)STEP_BATCH);
     if (want < 2 || nShots < 2 || !engine_batchable(c->eng)) return 0;
-    const int nb = ensure_lanes(c, nShots, true, want);
+    const int nb = ensure_lanes(c, nShots, true, true, want);
     return nb >= 2 ? nb : 0;
 }
 
@@ -512,11 +512,10 @@ static std::vector<std::pair<int, int>> shot_groups(int nShots, int nb) {
 
 // device bytes a lane needs for a shot: wavefield levels, secondary sources and, for Born, the history
 // (with shot windows set, of the widest window: a lane's buffers grow to the largest shot it runs)
-static int widest(const eio_ctx* c) {
-    return c->win_nx.empty() ? c->fd.p.nx : *std::max_element(c->win_nx.begin(), c->win_nx.end());
-}
 static size_t lane_bytes(const eio_ctx* c, bool born) {
-    const size_t n = (size_t)c->fd.p.nz * widest(c);
+    int nx = c->fd.p.nx;
+    if (!c->win_nx.empty()) nx = *std::max_element(c->win_nx.begin(), c->win_nx.end());
+    const size_t n = (size_t)c->fd.p.nz * nx;
     size_t b = sizeof(float) * n * 40;
     if (born) b += (size_t)2 * c->fd.p.nts * n * (engine_get_checkpoint(c->eng) ? 2 : 4);
     return b;
@@ -829,7 +828,7 @@ EIO_API int eio_born_shots_dev(eio_ctx* c, int adj, int nShots, float* const* sr
         if (!c || !srcDtw || !dm || !data || !srcPos || !nSrc || !recPos || !nRec || nShots < 1)
             throw Error(EIO_ERR_ARG, "null argument");
         const int nb = born_batch_width(c, nShots);
-        const int nl = nb ? nb : ensure_lanes(c, nShots, true);
+        const int nl = nb ? nb : ensure_lanes(c, nShots, true, true);
         std::vector<float*> lane_dm((size_t)5 * nl);
         for (int k = 0; k < nl; k++) {
             if (adj && k > 0) {   // the other lanes image into their own buffers, added below
@@ -1253,7 +1252,7 @@ static void nl_forward_batched(eio_ctx* c, int add, int nExp, int nModelExp, con
                                eio_sinterp* const* src, eio_sinterp* const* rec, int nRecGeom, size_t dslice,
                                size_t mslice) {
     const int nts = c->fd.p.nts;
-    const int nb = ensure_lanes(c, nExp, false, std::min(c->batch, (int)STEP_BATCH));
+    const int nb = ensure_lanes(c, nExp, false, false, std::min(c->batch, (int)STEP_BATCH));
     for (int s0 = 0; s0 < nExp; s0 += nb) {
         ShotGroup grp(c, s0, std::min(nb, nExp - s0), nExp, src, rec, nRecGeom);
         for (int i = 0; i < grp.cnt; i++) {
@@ -1297,7 +1296,7 @@ static int nl_forward_impl(eio_ctx* c, int add, int nExp, int nModelExp, const f
             nl_forward_batched(c, add, nExp, nModelExp, model, data, src, rec, nRecGeom, dslice, mslice);
             return;
         }
-        const int nl = ensure_lanes(c, nExp, false);
+        const int nl = ensure_lanes(c, nExp, false, true);
         std::vector<float*> tmp(nl);
         for (int k = 0; k < nl; k++) tmp[k] = add ? lane_staging(c, k, dslice) : nullptr;
         run_lanes(c, nl, nExp, [&](int k, Engine* eng, int e) {
@@ -1324,7 +1323,7 @@ static void nl_adjoint_batched(eio_ctx* c, int nExp, int nModelExp, float* model
                                eio_sinterp* const* src, eio_sinterp* const* rec, int nRecGeom, size_t dslice,
                                size_t mslice) {
     const int nts = c->fd.p.nts;
-    const int nb = ensure_lanes(c, nExp, false, std::min(c->batch, (int)STEP_BATCH));
+    const int nb = ensure_lanes(c, nExp, false, false, std::min(c->batch, (int)STEP_BATCH));
     for (int s0 = 0; s0 < nExp; s0 += nb) {
         ShotGroup grp(c, s0, std::min(nb, nExp - s0), nExp, src, rec, nRecGeom);
         for (int i = 0; i < grp.cnt; i++) grp.dp[i] = const_cast<float*>(data) + (size_t)(s0 + i) * dslice;
@@ -1362,7 +1361,7 @@ static int nl_adjoint_impl(eio_ctx* c, int add, int nExp, int nModelExp, float* 
             nl_adjoint_batched(c, nExp, nModelExp, model, data, src, rec, nRecGeom, dslice, mslice);
             return;
         }
-        const int nl = ensure_lanes(c, nExp, false);
+        const int nl = ensure_lanes(c, nExp, false, true);
         // constant source signal: every shot stacks into one model (nonlinearPropElasticShotsGpu.cpp:384-417),
         // here one partial stack per lane, added in lane order
         std::vector<std::vector<float>> slice(nl, std::vector<float>(mslice, 0.f));
@@ -1529,7 +1528,7 @@ static int eio_born_forward_impl(eio_ctx* c, int add, int nExp, const float* mod
             if ((size_t)5 * g.r[0]->nIrreg * nts != dslice) throw Error(EIO_ERR_ARG, "receiver counts differ");
         }
         const int nb = born_batch_width(c, nExp);
-        const int nl = nb ? nb : ensure_lanes(c, nExp, true);
+        const int nl = nb ? nb : ensure_lanes(c, nExp, true, true);
         for (int k = 0; k < nl; k++) engine_dm_upload(lane_engine(c, k), dm);   // stays on the device for every shot
         std::vector<float*> tmp(nl);
         for (int k = 0; k < nl; k++) tmp[k] = add ? lane_staging(c, k, dslice) : nullptr;
@@ -1627,7 +1626,7 @@ static int eio_born_adjoint_impl(eio_ctx* c, int add, int nExp, float* model, co
             if ((size_t)5 * g.r[0]->nIrreg * nts != dslice) throw Error(EIO_ERR_ARG, "receiver counts differ");
         }
         const int nb = born_batch_width(c, nExp);
-        const int nl = nb ? nb : ensure_lanes(c, nExp, true);
+        const int nl = nb ? nb : ensure_lanes(c, nExp, true, true);
         for (int k = 0; k < nl; k++) engine_dm_zero(lane_engine(c, k));   // each lane's shots accumulate on its device
         if (nb) {
             for (const auto& grp : shot_groups(nExp, nb)) {
@@ -1731,7 +1730,7 @@ static int eio_fwi_gradient_impl(eio_ctx* c, int nExp, int nModelExp, const floa
             if ((size_t)5 * g.s[0]->nIrreg * nts != mslice || (size_t)5 * g.r[0]->nIrreg * nts != dslice)
                 throw Error(EIO_ERR_ARG, "device counts differ between shots");
         }
-        const int nl = ensure_lanes(c, nExp, true);
+        const int nl = ensure_lanes(c, nExp, true, true);
         for (int k = 0; k < nl; k++) engine_dm_zero(lane_engine(c, k));
         std::vector<std::vector<float>> dtmp(nl), rtmp(nl);
         std::vector<double> phi(nExp, 0.0);

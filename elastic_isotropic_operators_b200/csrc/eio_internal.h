@@ -68,8 +68,6 @@ void engine_set_checkpoint(Engine* e, int mode);
 void engine_set_kernel(Engine* e, int kind, int tz, int cw, int cpr);
 void engine_pin_kernel(Engine* e);                            // the choice is the caller's: no resident loop
 void engine_copy_choice(Engine* to, const Engine* from);      // kernel choice of another engine of the grid
-// whether nonlinear propagations of `shots` shots at once on nx columns run as the resident loop
-bool engine_resident(const Engine* e, int nx, int shots);
 void engine_set_wait_limit(Engine* e, long long polls);   // < 0: the default
 void engine_share_medium(Engine* e, const Engine* from);   // e's kernels read from's medium arrays
 void engine_set_persistent(Engine* e, int mask);          // phases of the shot groups run as persistent loops

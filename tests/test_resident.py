@@ -186,3 +186,39 @@ def test_resident_beside_the_persistent_born_groups():
         for o in out[k]:
             for a, b in zip(o, ref[k]):
                 np.testing.assert_array_equal(a, b)
+
+
+UNTUNED = (1, 64, 8, 8)     # what eio_ctx_get_kernel says before any timing
+
+
+def _kernel(op):
+    v = [ctypes.c_int() for _ in range(4)]
+    _lib.check(op._L.eio_ctx_get_kernel(op.ctx, *[ctypes.byref(x) for x in v]))
+    return tuple(x.value for x in v)
+
+
+def test_lanes_choose_their_kernel_before_they_run():
+    # the saved wavefield's shot takes the step launches, on the second lane here: the first lane timed
+    # the kernels beforehand, alone, and both use its choice
+    w = synthetic.small(nts=40, nshots=4)
+    w.par.set("saveWavefield", "1")
+    w.par.set("wavefieldShotNumber", "1")
+    op = _pair(w)[0]
+    m, d = op.modelSpace(), op.dataSpace()
+    m.getNdArray()[...] = w.source_signal()[None]
+    op.forwardWavefield(False, m, d)
+    assert _kernel(op) != UNTUNED
+    ref = _run(op, w)[0]
+    np.testing.assert_array_equal(d.getNdArray(), ref)
+
+
+@pytest.mark.parametrize("nz,nx,shots,fwd,adj", [
+    (312, 520, 1, False, False), (312, 424, 3, False, True), (72, 104, 2, False, False), (600, 1000, 1, True, True)])
+def test_resident_calls_time_no_kernel(nz, nx, shots, fwd, adj):
+    w = synthetic.small(nz=nz, nx=nx, nts=5, nshots=shots)
+    for direction, timed in (("forward", fwd), ("adjoint", adj)):
+        op = _pair(w)[0]
+        m, d = op.modelSpace(), op.dataSpace()
+        m.getNdArray()[...] = w.source_signal()[None]
+        getattr(op, direction)(False, m, d)
+        assert (_kernel(op) != UNTUNED) == timed, direction
