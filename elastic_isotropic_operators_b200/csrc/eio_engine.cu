@@ -174,6 +174,7 @@ struct Engine {
     int kind = 1, tz = 64, cw = 8, cpr = 8;
     bool tuned = false;
     bool pinned = false;      // the kernel choice came from the caller: no resident loop
+    int peers = 1;            // engines that the current call runs side by side
     // resident time loop (eio_resident.cuh): shot table, step weights, edge slots, point tables
     DBuf res_shot, res_step, res_x, res_map, res_first[2], res_pt[2];
     // tensor maps of the sweep kernel (valid for mtz/mcw)
@@ -1322,6 +1323,36 @@ static bool res_points(const Engine* e, const ResPlan& p, const int* const pos[4
 // (eio_ctx_set_kernel), captured graphs and the free surface keep their launches
 static bool res_allowed(const Engine* e) { return !e->pinned && !e->use_graphs && !e->fs; }
 
+// Nonlinear propagations side by side on a device.  Resident launches take
+// turns, step launches of small grids overlap: two of a kind are still faster
+// resident, more are not.  Microseconds a shot and fine step, resident / step
+// launches, contexts on host threads: 72 x 104 two 2.67 / 3.01, four 2.66 / 1.62;
+// 312 x 520 two 3.98 / 4.45, four 4.02 / 2.56; four lanes of one call 2.84 / 1.68
+// and 4.17 / 2.64.
+constexpr int RES_AT_ONCE = 2;
+struct NlFlight {
+    std::atomic<int>& n;
+    const int now;          // propagations in flight on the device, this one too
+    explicit NlFlight(int device) : n(count(device)), now(++n) {}
+    ~NlFlight() { --n; }
+    NlFlight(const NlFlight&) = delete;
+    NlFlight& operator=(const NlFlight&) = delete;
+    static std::atomic<int>& count(int device) {
+        static std::atomic<int> c[64];
+        return c[device & 63];
+    }
+};
+void engine_set_peers(Engine* e, int n) { e->peers = n; }
+
+// A small-grid call that gives way to others and has no kernel choice yet takes
+// the tile kernel: timed among the others' work, chance makes the choice (eight
+// contexts of 312 x 520: 3.1 us a shot and step, with the tile kernel 2.2).
+static void choose_kernel(Engine* e, bool gave_way) {
+    if (e->tuned) return;
+    if (gave_way) e->kind = 0;
+    else engine_autotune(e);
+}
+
 // One nonlinear propagation of nb shots (engines es, all of the first one's
 // device, grid height and time axis; each with its own window) as one launch.
 struct Resident {
@@ -1335,20 +1366,27 @@ struct Resident {
 
     Resident(Engine* const* engines, int n) : es(engines), nb(n), inj(n), ext(n), sh(n) {}
 
+    // within the resident loop's sizes, and free to take it
+    bool small(int adj) const {
+        long long cells = 0;
+        for (int i = 0; i < nb; i++) {
+            if (!res_allowed(es[i])) return false;
+            cells += es[i]->n;
+        }
+        return cells <= RES_CELLS[adj];
+    }
+
     // The cheapest plan with all shots side by side whose point buffers fit
     // too; false: no such plan, or not the better way.  g: acquisition per
     // shot; the adjoint injects at the receivers.
     bool plan(const ShotGeom* g, int adj) {
         Engine* e0 = es[0];
+        if (!small(adj) || e0->nsm < nb) return false;
         int nx = 0, nx_min = 1 << 30;
-        long long cells = 0;
         for (int i = 0; i < nb; i++) {
-            if (!res_allowed(es[i])) return false;
             nx = std::max(nx, es[i]->nx);
             nx_min = std::min(nx_min, es[i]->nx);
-            cells += es[i]->n;
         }
-        if (cells > RES_CELLS[adj] || e0->nsm < nb) return false;
         int tried = 0;
         for (const ResPlan& c : res_plans(e0->nz, nx, nx_min, e0->nsm / nb)) {
             if (tried++ == 6) break;
@@ -1462,7 +1500,10 @@ void engine_nl(Engine* e, int adj, float* const model[5], float* const data[5], 
     EIO_CUDA(cudaSetDevice(e->device));
     if (wfld && e->windowed) throw Error(EIO_ERR_UNSUPPORTED, "saved wavefields cover the whole grid: no shot windows");
     PointList src, rec;
-    if (!wfld && res_allowed(e)) {
+    const NlFlight flight(e->device);
+    const bool small = !wfld && res_allowed(e) && e->n <= RES_CELLS[adj];
+    const bool way = std::max(flight.now, e->peers) > RES_AT_ONCE;   // gives way
+    if (small && !way) {
         build_points(e, g.srcPos, g.nSrc, src);
         build_points(e, g.recPos, g.nRec, rec);
         Resident r(&e, 1);
@@ -1481,7 +1522,7 @@ void engine_nl(Engine* e, int adj, float* const model[5], float* const data[5], 
             return;
         }
     }
-    if (!e->tuned) engine_autotune(e);   // the choice serves the Born operators too: timed without the free surface
+    choose_kernel(e, small && way);   // it serves the Born operators too: timed without the free surface
     FsScope fs_scope(e);
     err_reset(e);
     build_points(e, g.srcPos, g.nSrc, src);
@@ -2356,9 +2397,11 @@ void engine_nl_shots_batch(Engine* const* es, int nb, int adj, float* const* mod
     Engine* e0 = es[0];
     EIO_CUDA(cudaSetDevice(e0->device));
     Resident res(es, nb);
-    const bool resident = res.plan(g, adj);
+    const NlFlight flight(e0->device);
+    const bool way = flight.now > RES_AT_ONCE;
+    const bool resident = !way && res.plan(g, adj);
     if (!resident) {
-        if (!e0->tuned) engine_autotune(e0);
+        choose_kernel(e0, way && res.small(adj));
         for (int i = 1; i < nb; i++) engine_copy_choice(es[i], e0);   // one tile geometry
     }
     const int minb = (e0->kind == 3 || e0->kind == 5) ? 4 : 3;

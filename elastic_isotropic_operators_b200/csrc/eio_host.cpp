@@ -470,6 +470,7 @@ static void run_lanes(eio_ctx* c, int n, int nShots, F&& f) {
         for (int s = 0; s < nShots; s++) f(0, c->eng, s);
         return;
     }
+    for (int k = 0; k < n; k++) engine_set_peers(lane_engine(c, k), n);
     std::vector<std::exception_ptr> err(n);
     std::vector<std::thread> th;
     th.reserve(n);
@@ -482,6 +483,7 @@ static void run_lanes(eio_ctx* c, int n, int nShots, F&& f) {
             }
         });
     for (auto& t : th) t.join();
+    for (int k = 0; k < n; k++) engine_set_peers(lane_engine(c, k), 1);
     for (auto& x : err)
         if (x) std::rethrow_exception(x);
 }

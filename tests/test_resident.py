@@ -222,3 +222,27 @@ def test_resident_calls_time_no_kernel(nz, nx, shots, fwd, adj):
         m.getNdArray()[...] = w.source_signal()[None]
         getattr(op, direction)(False, m, d)
         assert (_kernel(op) != UNTUNED) == timed, direction
+
+
+def _resident(op, call):
+    """Whether the call's fine steps were one launch (counters: launches of any kind, fine steps)."""
+    n, s = ctypes.c_longlong(), ctypes.c_longlong()
+    _lib.check(op._L.eio_ctx_stats(op.ctx, 0, 1, None, None, None))
+    call()
+    _lib.check(op._L.eio_ctx_stats(op.ctx, 0, 0, ctypes.byref(n), ctypes.byref(s), None))
+    assert s.value > 0
+    return n.value < s.value
+
+
+@pytest.mark.parametrize("lanes,resident", [(2, True), (3, False), (4, False)])
+def test_more_than_two_lanes_keep_their_overlapping_launches(lanes, resident):
+    w = synthetic.small(nts=60, nshots=4)
+    op = _pair(w)[0]
+    ref = _run(op, w)
+    op.setShotBatch(1)
+    op.setLanes(lanes)
+    assert _resident(op, lambda: _run(op, w)) == resident
+    for a, b in zip(_run(op, w), ref):
+        np.testing.assert_allclose(a, b, rtol=0, atol=1e-6 * np.abs(b).max())
+    op.setLanes(1)
+    assert _resident(op, lambda: _run(op, w))
