@@ -1015,7 +1015,7 @@ void engine_set_kernel(Engine* e, int kind, int tz, int cw, int cpr) {
     e->tuned = true;
 }
 
-void engine_pin_kernel(Engine* e) { e->pinned = true; }
+void engine_pin_kernel(Engine* e, bool pin) { e->pinned = pin; }
 void engine_copy_choice(Engine* to, const Engine* from) {
     to->kind = from->kind; to->tz = from->tz; to->cw = from->cw; to->cpr = from->cpr;
     to->tuned = from->tuned;

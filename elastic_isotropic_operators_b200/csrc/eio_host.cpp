@@ -712,7 +712,7 @@ EIO_API int eio_ctx_set_kernel(eio_ctx* c, int kind, int tz, int cw, int cpr) {
     return guarded([&] {
         if (!c) throw Error(EIO_ERR_ARG, "null context");
         engine_set_kernel(c->eng, kind, tz, cw, cpr);
-        engine_pin_kernel(c->eng);
+        engine_pin_kernel(c->eng, true);
         for (Engine* e : c->extra) engine_copy_choice(e, c->eng);
     });
 }
@@ -746,6 +746,7 @@ EIO_API int eio_ctx_autotune(eio_ctx* c, int* kind, int* tz, int* cw, int* cpr) 
     return guarded([&] {
         if (!c) throw Error(EIO_ERR_ARG, "null context");
         engine_autotune(c->eng);
+        engine_pin_kernel(c->eng, false);   // the choice is the library's again
         for (Engine* e : c->extra) engine_copy_choice(e, c->eng);
         engine_get_kernel(c->eng, kind, tz, cw, cpr);
     });

@@ -66,7 +66,7 @@ void engine_set_medium(Engine* e, const FdParam& fd);
 void engine_set_checkpoint(Engine* e, int mode);
 // step-kernel selection: kind 0 tile kernel, 1 TMA sweep (tz, cw, cpr); autotune times the candidates
 void engine_set_kernel(Engine* e, int kind, int tz, int cw, int cpr);
-void engine_pin_kernel(Engine* e);                            // the choice is the caller's: no resident loop
+void engine_pin_kernel(Engine* e, bool pin);                  // the choice is the caller's: no resident loop
 void engine_set_peers(Engine* e, int n);                      // engines that the current call runs side by side
 void engine_copy_choice(Engine* to, const Engine* from);      // kernel choice of another engine of the grid
 void engine_set_wait_limit(Engine* e, long long polls);   // < 0: the default

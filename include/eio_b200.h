@@ -175,8 +175,12 @@ void *eio_ctx_stream(eio_ctx *c);
  * launch (the tile widened by the stencil radius, four wavefield levels), kind 3
  * for the steps that run alone (free surface, saved wavefields, the last
  * coarse interval of a Born source wavefield, running-sum epilogues).  By
- * default the first propagation of a context times every candidate on its
- * grid (eio_ctx_autotune) and keeps the fastest. */
+ * default the first propagation of a context that needs one times every
+ * candidate on its grid and keeps the fastest.  The nonlinear operators need
+ * none on small grids (all shots of a call together up to 420000 cells forward):
+ * every fine step runs in one launch, with the same bits.  A kernel set here
+ * is launched once per fine step on every grid, until eio_ctx_autotune times the
+ * candidates and gives the choice back to the library. */
 int eio_ctx_set_kernel(eio_ctx *c, int kind, int tz, int cw, int cpr);
 int eio_ctx_get_kernel(const eio_ctx *c, int *kind, int *tz, int *cw, int *cpr);
 int eio_ctx_autotune(eio_ctx *c, int *kind, int *tz, int *cw, int *cpr);

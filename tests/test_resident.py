@@ -246,3 +246,11 @@ def test_more_than_two_lanes_keep_their_overlapping_launches(lanes, resident):
         np.testing.assert_allclose(a, b, rtol=0, atol=1e-6 * np.abs(b).max())
     op.setLanes(1)
     assert _resident(op, lambda: _run(op, w))
+
+
+def test_autotune_takes_the_choice_back():
+    w = synthetic.small(nts=60, nshots=1)
+    op = _pair(w)[1]
+    assert not _resident(op, lambda: _run(op, w))      # the caller's kernel
+    _lib.check(op._L.eio_ctx_autotune(op.ctx, None, None, None, None))
+    assert _resident(op, lambda: _run(op, w))
