@@ -1082,9 +1082,9 @@ __global__ void __launch_bounds__(T_THREADS, CPS) k_conv_tma(const __grid_consta
 // k_conv_halo: the forward and data-gradient convolutions of wide images (128
 // pixels of a row per tile) with one copy of the input for all nine taps.
 // k_conv_tma fetches a box per tap, nine times the tile, in rows of 32 to 128
-// bytes, and TMA takes about eight cycles a row whatever its length (250 rows
-// per microsecond and SM here); the full-resolution layers of 16 to 96 channels
-// ran at that rate, tensor pipe and DRAM below 10 %.  Here a stage is the
+// bytes, and an SM gets through one box row in three to four cycles whatever its
+// length (16 -> 32 and 64 -> 32 channels at 16 images of 256 x 256); that is what
+// its full-resolution layers of few channels take.  Here a stage is the
 // tile's R image rows with their halo, (R + 2) x 130 pixels of every channel
 // block (box {cb, 130, R + 2}: 2 box rows per output pixel at R = 2 against 9),
 // and a tap is a whole number of pixel rows into it: the K-major operand of
@@ -1092,11 +1092,11 @@ __global__ void __launch_bounds__(T_THREADS, CPS) k_conv_tma(const __grid_consta
 // swizzle being a function of the shared-memory address.  The weights (9 cin x
 // cout) stay in shared memory for all tiles of the persistent CTA.  The sums
 // run over taps, channel blocks and K steps in k_conv_tma's order: same bits.
-// Measured, 16 images of 256 x 256 (B200, k_conv_tma with four CTAs per SM against
-// this): 16 -> 32 channels 93 / 40 us (15 at the HBM rate), 32 -> 32 126 / 60,
-// 32 -> 16 122 / 58, 32 -> 96 171 / 105, 64 -> 64 at 128 x 128 60 / 48; 96 -> 32,
-// whose three blocks leave one row a tile and one CTA an SM, 324 / 316.  Copies
-// by cp.async warps in place of TMA were slower (32 -> 32 88 us).
+// Measured, 16 images of 256 x 256, warm (B200, k_conv_tma with up to four CTAs per
+// SM against this): 16 -> 32 channels 112 / 35 us (15 at the HBM rate), 32 -> 32 98 / 56,
+// 32 -> 16 79 / 54, 32 -> 96 172 / 101, 64 -> 64 at 128 x 128 46 / 43.  96 -> 32, whose
+// three blocks leave one row a tile and one CTA an SM, 201 / 313: halo_pays leaves it
+// to k_conv_tma.  Copies by cp.async warps in place of TMA were slower (32 -> 32 88 us).
 constexpr int HALO_W = 128, HALO_P = HALO_W + 2;
 
 struct ConvHalo {
@@ -1303,8 +1303,7 @@ __global__ void __launch_bounds__(T_THREADS) k_conv_halo(const __grid_constant__
 // ---------------------------------------------------------------------------
 // k_wgrad_halo: the weight gradients of wide images with the same halo stages.
 // k_conv_tma fetches the nine shifted copies of x, and dz once per 128 rows of
-// the result: 12 box rows a pixel at 32 channels (27 at 96), at TMA's rate of
-// rows.  Here a stage is R image rows of x with their halo ((R + 2) x 136 pixels
+// the result: 12 box rows a pixel at 32 channels (27 at 96).  Here a stage is R image rows of x with their halo ((R + 2) x 136 pixels
 // per channel block) and R x 128 pixels of dz: 3 box rows a pixel.  The product
 // of column offset dx is one MN-major operand whose blocks of cb channels are the
 // image rows below each other (block stride one row of the slab): 128 / cb
@@ -1312,8 +1311,9 @@ __global__ void __launch_bounds__(T_THREADS) k_conv_halo(const __grid_constant__
 // accumulator per channel block, dx and group of vertical taps stays in tensor
 // memory over all tiles of the persistent CTA, which writes one partial result;
 // k_sum_splits adds them in order, so the sum is reproducible.
-// Measured, 16 images of 256 x 256 (B200, k_conv_tma with four CTAs per SM against
-// this): 16 -> 32 channels 249 / 124 us, 32 -> 32 261 / 126, 32 -> 16 263 / 124.
+// Measured, 16 images of 256 x 256, warm (B200, k_conv_tma with up to four CTAs per SM
+// against this): 16 -> 32 channels 247 / 121 us, 32 -> 32 260 / 122, 32 -> 16 260 / 120,
+// 64 -> 64 353 / 292, 96 -> 32 605 / 555.
 constexpr int WG_P = 136;      // slab row: 128 pixels, their halo, rounded to the swizzle pattern
 
 struct WgradHalo {
@@ -1708,7 +1708,18 @@ constexpr size_t H_SM = 227 * 1024;     // shared memory of an SM that CTAs can 
 
 // the deepest plan that fits: two rows per tile where the height allows, two
 // to four stages, as many CTAs per SM as tensor and shared memory hold
-bool halo_plan(int h, int w, int cin, int cout, HaloPlan* p)
+//
+// Where the plan pays (time over k_conv_tma's at 1 to 55 tiles an SM, 256-pixel rows): with two or more CTAs
+// per SM always (1.00 falling to 0.33).  With one, and one tile each, too (0.64 to 0.87: one copy's latency
+// instead of nine).  Over several tiles one CTA leaves the SM waiting for its copies, unless the tile's
+// MMAs are long enough to cover them: two rows at 48 or 64 output channels (0.65 to 0.95) or 96 (0.47 to
+// 1.01); not 64 -> 32 (1.06 to 1.21), 96 -> 32 (1.33 to 1.57) or one row of 64 -> 64 (1.17 to 1.22), whose
+// k_conv_tma has three or four CTAs per SM.
+bool halo_pays(const HaloPlan& p, int bn, long long tiles)
+{
+    return p.ctas > 1 || tiles <= g_sms() || bn == 96 || (bn == 64 && p.r == 2);
+}
+bool halo_plan(int n, int h, int w, int cin, int cout, HaloPlan* p)
 {
     const int cb = chan_block(cin), bn = tma_bn(cout);
     if (g_use_tma < 3 || !cb || w % HALO_W || cout % 16 || cout > bn || bn > 96) return false;
@@ -1727,7 +1738,7 @@ bool halo_plan(int h, int w, int cin, int cout, HaloPlan* p)
             p->ctas = ctas;
             p->stages = (int)std::min<long long>(st, 4);
             p->smem = most;
-            return true;
+            return halo_pays(*p, bn, (long long)n * (h / r) * (w / HALO_W));
         }
     }
     return false;
@@ -1803,6 +1814,8 @@ bool wgrad_plan(int n, int h, int w, int cin, int cout, WgradPlan* p)
 {
     const int cb = chan_block(cin);
     if (g_use_tma < 3 || !cb || w % HALO_W || (cout != 16 && cout != 32 && cout != 64)) return false;
+    // 48 and 80 input channels, in blocks of 16: 1.13 to 1.41 times k_conv_tma's time at every size
+    if (cb == 16 && cin > 16) return false;
     const int cpt = cin / cb, per = G_BM / cb, cols = std::max(cout, 32);
     p->ngrp = (3 + per - 1) / per;
     const int used = cpt * 3 * p->ngrp * cols;
@@ -1811,14 +1824,17 @@ bool wgrad_plan(int n, int h, int w, int cin, int cout, WgradPlan* p)
     // the last operand reads (and leaves out) rows past the last slab
     const size_t tail = (size_t)(p->ngrp * per - 3) * WG_P * cb * 2;
     for (int r = h % 2 ? 1 : 2; r >= 1; r--) {
-        // a CTA's one partial result pays off over several tiles; k_conv_tma splits small images finer
         const long long tiles = (long long)n * (h / r) * (w / HALO_W);
-        if (tiles < 2LL * g_sms() || tiles > (1LL << 30)) continue;
+        if (tiles > (1LL << 30)) continue;
         const size_t stage = (size_t)wgrad_dz(cpt, cb, r) + (size_t)r * HALO_W * cout * 2;
         for (int ctas = std::min(4, 512 / talloc); ctas >= 1; ctas--) {
             const size_t most = H_SM / ctas - 2048;
             const long long st = ((long long)most - 1024 - (long long)tail) / (long long)stage;
             if (st < 2 || (st < 3 && ctas > 2)) continue;
+            // A CTA's one partial result pays off over several tiles; k_conv_tma splits small images finer.
+            // Time over k_conv_tma's: two or more CTAs per SM 0.93 to 1.04 at 3.5 rows of 128 pixels an SM, 0.62
+            // to 0.85 at 7; one 0.93 to 1.18 at 7, 0.84 to 0.98 at 14.
+            if (tiles * r < (ctas > 1 ? 4LL : 12LL) * g_sms()) return false;
             p->r = r;
             p->stages = (int)std::min<long long>(st, 4);
             p->smem = most;
@@ -1952,7 +1968,7 @@ void unet_conv3x3(int n, int h, int w, int cin, int cout, const void* x, const v
     check16opt(y32, "FP32 output");
     check16opt(y16, "BF16 output");
     HaloPlan hp;
-    if (halo_plan(h, w, cin, cout, &hp)) {
+    if (halo_plan(n, h, w, cin, cout, &hp)) {
         conv_halo(n, h, w, cin, cout, x, wt, y32, y16, relu, hp, static_cast<cudaStream_t>(stream));
         return;
     }

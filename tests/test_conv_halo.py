@@ -20,7 +20,10 @@ def _p(t):
 
 @pytest.mark.parametrize("n,h,w,cin,cout", [
     (1, 1, 128, 16, 16), (2, 5, 128, 16, 32), (1, 6, 256, 32, 32), (3, 4, 384, 32, 16), (1, 7, 256, 48, 32),
-    (1, 4, 128, 96, 32), (2, 2, 256, 32, 96), (1, 8, 128, 64, 64), (1, 40, 1024, 32, 48), (20, 16, 256, 16, 32)])
+    (1, 4, 128, 96, 32), (2, 2, 256, 32, 96), (1, 8, 128, 64, 64), (1, 40, 1024, 32, 48), (20, 16, 256, 16, 32),
+    # one CTA an SM: a tile each, and two or more
+    (1, 37, 512, 96, 32), (1, 75, 256, 96, 32), (2, 148, 128, 64, 32), (2, 149, 128, 64, 64), (4, 76, 256, 64, 64),
+    (1, 149, 128, 64, 96), (3, 100, 128, 48, 48)])
 def test_halo_convolution_equals_the_copy_loop(n, h, w, cin, cout):
     torch = pytest.importorskip("torch")
     L = _lib.lib()
@@ -109,9 +112,12 @@ def test_loss_and_its_derivative(npix, c, nc):
     assert abs(loss.item() - ref) <= 1e-12 * ref
 
 
-@pytest.mark.parametrize("n,h,w,cin,cout", [      # at least two tiles per SM, else the split GEMM runs
-    (300, 1, 128, 16, 16), (300, 1, 128, 16, 64), (60, 5, 128, 32, 64), (100, 5, 128, 16, 32), (5, 120, 128, 32, 32), (4, 50, 384, 32, 16), (3, 151, 256, 48, 32),
-    (2, 150, 128, 96, 32), (2, 302, 128, 64, 64), (2, 101, 256, 64, 16), (20, 32, 256, 32, 32), (1, 6, 256, 32, 32)])
+@pytest.mark.parametrize("n,h,w,cin,cout", [      # small images take the split GEMM
+    (300, 1, 128, 16, 16), (100, 5, 128, 16, 32), (5, 120, 128, 32, 32), (4, 50, 384, 32, 16), (3, 151, 256, 48, 32),
+    (2, 150, 128, 96, 32), (2, 302, 128, 64, 64), (2, 101, 256, 64, 16), (20, 32, 256, 32, 32), (1, 6, 256, 32, 32),
+    # both sides of the rule: 4 rows of 128 pixels an SM, 12 where one CTA fits; dz after slabs of odd size
+    (592, 1, 128, 16, 64), (591, 1, 128, 16, 64), (120, 5, 128, 32, 64), (37, 16, 128, 32, 16), (37, 16, 128, 16, 32),
+    (8, 111, 256, 64, 64), (6, 148, 256, 64, 32), (7, 127, 256, 96, 32), (6, 148, 256, 32, 64), (592, 1, 128, 48, 32)])
 def test_halo_weight_gradient(n, h, w, cin, cout):
     """Against FP64 products of the same BF16 values: FP32 sums of n h w terms, relative L2 <= 1e-5 (as the
     other weight-gradient kernels); reproducible."""
@@ -138,7 +144,7 @@ def test_halo_kernels_on_threads():
     run them at once, each on its own stream: every launch is accepted and gives the bits of a serial run."""
     torch = pytest.importorskip("torch")
     L = _lib.lib()
-    n, h, w, cout = 300, 1, 128, 32
+    n, h, w, cout = 1800, 1, 128, 32
     bf = lambda *s: torch.randn(*s, device="cuda").to(torch.bfloat16)  # noqa: E731
     jobs = []
     for cin in (16, 32, 64):
