@@ -1389,7 +1389,10 @@ struct Resident {
         }
         int tried = 0;
         for (const ResPlan& c : res_plans(e0->nz, nx, nx_min, e0->nsm / nb)) {
-            if (tried++ == 6) break;
+            // Two columns a unit leave the adjoint, which moves the fields themselves through L2, at its step
+            // launches' time or above (calls of 157 k to 200 k cells 0.91 to 1.12 of it, above to 1.30); with
+            // one it takes 0.66 to 0.97, up to 180 k cells.
+            if (tried++ == 6 || (adj && c.CB != 1)) break;
             p = c;
             inj_cap = ext_cap = 0;
             for (int i = 0; i < nb; i++) {
@@ -1483,8 +1486,8 @@ struct Resident {
         for (int k = 0; k < 4; k++) { a.cz[k] = e->zc[k]; a.cx[k] = e->xc[k]; }
         a.err = static_cast<int*>(e->err.p);
         a.wait_limit = e->wait_limit;
-        const void* fn = adj ? (p.CB == 1 ? (const void*)k_resident<1, 1> : (const void*)k_resident<1, 2>)
-                             : (p.CB == 1 ? (const void*)k_resident<0, 1> : (const void*)k_resident<0, 2>);
+        const void* fn = adj ? (const void*)k_resident<1, 1>
+                             : p.CB == 1 ? (const void*)k_resident<0, 1> : (const void*)k_resident<0, 2>;
         EIO_CUDA(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)RES_SMEM));
         void* args[] = {&a};
         launch_cooperative(e, fn, nb * p.ctas(), p.threads + p.serv, args, res_smem(p.mq, p.mx, inj_cap, ext_cap));

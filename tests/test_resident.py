@@ -213,7 +213,9 @@ def test_lanes_choose_their_kernel_before_they_run():
 
 
 @pytest.mark.parametrize("nz,nx,shots,fwd,adj", [
-    (312, 520, 1, False, False), (312, 424, 3, False, True), (72, 104, 2, False, False), (600, 1000, 1, True, True)])
+    (312, 520, 1, False, False), (312, 424, 3, False, True), (72, 104, 2, False, False), (600, 1000, 1, True, True),
+    # the adjoint where its plan has two columns a unit: not faster than its launches
+    (312, 600, 1, False, True), (56, 3400, 1, False, True), (1000, 200, 1, False, True), (72, 344, 8, False, True)])
 def test_resident_calls_time_no_kernel(nz, nx, shots, fwd, adj):
     w = synthetic.small(nz=nz, nx=nx, nts=5, nshots=shots)
     for direction, timed in (("forward", fwd), ("adjoint", adj)):
