@@ -266,7 +266,7 @@ __global__ void __launch_bounds__(RES_THREADS, 1) k_resident(const __grid_consta
             float* d = pin + pt * 80 + par * 40 + f * 8 + j;
             const float* s = sh.inj_sig[f] + (long long)w.inj_t * sh.inj_ld[f] + col;
             cp_async4(d, s);
-            cp_async4(d + 4, w.iw1 != 0.f ? s + sh.inj_ld[f] : s);   // a last row is never read past
+            cp_async4(d + 4, s + sh.inj_ld[f]);      // inj_t is at most the last row but one
         }
     };
     auto slot = [](int kind, int code) {             // shared field of an edge entry

@@ -256,3 +256,22 @@ def test_autotune_takes_the_choice_back():
     assert not _resident(op, lambda: _run(op, w))      # the caller's kernel
     _lib.check(op._L.eio_ctx_autotune(op.ctx, None, None, None, None))
     assert _resident(op, lambda: _run(op, w))
+
+
+@pytest.mark.parametrize("value", [np.nan, np.inf])
+def test_non_finite_samples_spread_as_with_step_launches(value):
+    # a sample is part of every fine step between its neighbours, also where its time weight is zero
+    w = synthetic.small(nts=60, nshots=1)
+    out = []
+    for op in _pair(w):
+        m, d, a, b = op.modelSpace(), op.dataSpace(), op.modelSpace(), op.dataSpace()
+        m.getNdArray()[...] = w.source_signal()[None]
+        m.getNdArray().reshape(5, -1)[2, 30] = value
+        op.forward(False, m, d)
+        b.getNdArray()[...] = 1.0
+        b.getNdArray().reshape(5, 20, 60)[3, 7, 25] = value
+        op.adjoint(False, a, b)
+        out.append((d.getNdArray().copy(), a.getNdArray().copy()))
+    for got, ref in zip(*out):
+        assert 0 < np.isfinite(ref).sum() < ref.size
+        np.testing.assert_array_equal(got, ref)
