@@ -1402,9 +1402,36 @@ struct Resident {
                 inj_cap = std::max(inj_cap, inj[i].cap);
                 ext_cap = std::max(ext_cap, ext[i].cap);
             }
-            if (res_smem(p.mq, p.mx, inj_cap, ext_cap) <= RES_SMEM) return true;
+            if (res_smem(p.mq, p.mx, inj_cap, ext_cap) <= RES_SMEM) return reserve();
         }
         return false;
+    }
+
+    // The plan's device buffers (the edge slots are some MB).  False where they do not fit: the step launches,
+    // which need none of them, may still.
+    bool reserve() {
+        Engine* e0 = es[0];
+        try {
+            e0->res_x.ensure(sizeof(uint4) * slots() * nb);
+            e0->res_shot.ensure(sizeof(ResShot) * nb);
+            e0->res_step.ensure(sizeof(ResStep) * (size_t)(e0->nts - 1) * e0->S);
+            for (int i = 0; i < nb; i++)
+                for (int k = 0; k < 2; k++) {
+                    const ResPoints& r = k ? ext[i] : inj[i];
+                    if (!r.any) continue;
+                    if (k == 0) es[i]->res_map.ensure(sizeof(short) * r.map.size());
+                    es[i]->res_first[k].ensure(sizeof(int) * r.first.size());
+                    es[i]->res_pt[k].ensure(sizeof(ResPoint) * r.pt.size());
+                }
+        } catch (const Error& x) {
+            if (x.code != EIO_ERR_NOMEM) throw;
+            for (int i = 0; i < nb; i++)
+                for (DBuf* b : {&es[i]->res_x, &es[i]->res_shot, &es[i]->res_step, &es[i]->res_map, &es[i]->res_first[0],
+                                &es[i]->res_first[1], &es[i]->res_pt[0], &es[i]->res_pt[1]})
+                    b->release();
+            return false;
+        }
+        return true;
     }
 
     // edge slots of one shot, in uint4
@@ -1414,7 +1441,6 @@ struct Resident {
     // the first engine's stream is to wait for the others before run()
     void prepare() {
         Engine* e0 = es[0];
-        e0->res_x.ensure(sizeof(uint4) * slots() * nb);
         for (int i = 0; i < nb; i++) {
             Engine* e = es[i];
             ResShot& s = sh[i];

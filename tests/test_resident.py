@@ -275,3 +275,23 @@ def test_non_finite_samples_spread_as_with_step_launches(value):
     for got, ref in zip(*out):
         assert 0 < np.isfinite(ref).sum() < ref.size
         np.testing.assert_array_equal(got, ref)
+
+
+def test_resident_without_memory_for_its_slots_takes_the_step_launches():
+    # 6 MB of edge slots, and a context that has no more than its step launches needed
+    w = synthetic.small(nz=312, nx=520, nts=20, nshots=1)
+    op = _pair(w)[1]
+    ref = _run(op, w)
+    L = op._L
+    _lib.check(L.eio_ctx_autotune(op.ctx, None, None, None, None))     # no longer pinned
+    used = ctypes.c_longlong()
+    try:
+        _lib.check(L.eio_get_device_memory_used(ctypes.byref(used)))
+        _lib.check(L.eio_set_device_memory_cap(used.value + (1 << 20)))
+        got = []
+        assert not _resident(op, lambda: got.extend(_run(op, w)))
+        for a, b in zip(got, ref):
+            np.testing.assert_allclose(a, b, rtol=0, atol=1e-6 * np.abs(b).max())
+    finally:
+        _lib.check(L.eio_set_device_memory_cap(0))
+    assert _resident(op, lambda: _run(op, w))
