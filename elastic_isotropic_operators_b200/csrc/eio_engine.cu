@@ -1528,23 +1528,20 @@ struct Resident {
 void engine_nl(Engine* e, int adj, float* const model[5], float* const data[5], const ShotGeom& g, float* wfld) {
     EIO_CUDA(cudaSetDevice(e->device));
     if (wfld && e->windowed) throw Error(EIO_ERR_UNSUPPORTED, "saved wavefields cover the whole grid: no shot windows");
-    PointList src, rec;
     const NlFlight flight(e->device);
     const bool small = !wfld && res_allowed(e) && e->n <= RES_CELLS[adj];
     const bool way = std::max(flight.now, e->peers) > RES_AT_ONCE;   // gives way
     if (small && !way) {
-        build_points(e, g.srcPos, g.nSrc, src);
-        build_points(e, g.recPos, g.nRec, rec);
         Resident r(&e, 1);
         if (r.plan(&g, adj)) {
             err_reset(e);
             if (adj) zero_wavefields(e);
-            stage_in(e, adj ? data : model, adj ? rec.ld : src.ld, e->nts, e->sig_in);
-            zero_out(e, adj ? src.ld : rec.ld, e->nts, e->sig_out);
+            stage_in(e, adj ? data : model, r.inj[0].ld, e->nts, e->sig_in);
+            zero_out(e, r.ext[0].ld, e->nts, e->sig_out);
             r.prepare();
             r.run(adj);
             check_launch();
-            stage_out(e, adj ? src.ld : rec.ld, e->nts, e->sig_out, adj ? model : data);
+            stage_out(e, r.ext[0].ld, e->nts, e->sig_out, adj ? model : data);
             EIO_CUDA(cudaStreamSynchronize(e->st));
             stats_flush(e);
             err_check(e);
@@ -1554,6 +1551,7 @@ void engine_nl(Engine* e, int adj, float* const model[5], float* const data[5], 
     choose_kernel(e, small && way);   // it serves the Born operators too: timed without the free surface
     FsScope fs_scope(e);
     err_reset(e);
+    PointList src, rec;
     build_points(e, g.srcPos, g.nSrc, src);
     build_points(e, g.recPos, g.nRec, rec);
     StepArgs a = base_args(e);
