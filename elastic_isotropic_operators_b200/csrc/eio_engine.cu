@@ -176,7 +176,7 @@ struct Engine {
     bool pinned = false;      // the kernel choice came from the caller: no resident loop
     int peers = 1;            // engines that the current call runs side by side
     // resident time loop (eio_resident.cuh): shot table, step weights, edge slots, point tables
-    DBuf res_shot, res_step, res_x, res_map, res_first[2], res_pt[2];
+    DBuf res_x, res_tab;
     // tensor maps of the sweep kernel (valid for mtz/mcw)
     int mtz = -1, mcw = -1;
     CUtensorMap mwf_halo[10], mwf_int[10], mpar_halo[5], mpar_int[5];
@@ -415,8 +415,7 @@ void engine_destroy(Engine* e) {
     DBuf* all[] = {&e->dampz, &e->dampx, &e->inj_ts, &e->inj_ent, &e->inj_hts, &e->inj_hent, &e->ext_ts, &e->ext_ent,
                    &e->W, &e->err, &e->wsave,
                    &e->Wq, &e->wscale, &e->wstage, &e->wpmax, &e->dampz_fs, &e->fsc, &e->dampx_w,
-                   &e->res_shot, &e->res_step, &e->res_x, &e->res_map, &e->res_first[0],
-                   &e->res_first[1], &e->res_pt[0], &e->res_pt[1]};
+                   &e->res_x, &e->res_tab};
     for (DBuf* b : all) b->release();
     for (int k = 0; k < 4; k++) {
         e->rint[k].slot.release(); e->rint[k].w.release(); e->rint[k].start.release(); e->rint[k].ent.release();
@@ -1066,7 +1065,7 @@ void engine_get_kernel(const Engine* e, int* kind, int* tz, int* cw, int* cpr) {
     if (cpr) *cpr = tiled(e->kind) ? 0 : e->cpr;
 }
 
-static void zero_wavefields(Engine* e);
+static void zero_wavefields(Engine* e, int fields = 20);
 
 // Times every candidate on a few forward and adjoint fine steps of this grid
 // (no sparse points; the step cost does not depend on the field values) and
@@ -1129,8 +1128,8 @@ void engine_autotune(Engine* e) {
     if (flag) throw Error(EIO_ERR_TIMEOUT, "a TMA pipeline wait timed out while tuning");
 }
 
-static void zero_wavefields(Engine* e) {
-    for (int f = 0; f < 20; f++) EIO_CUDA(cudaMemsetAsync(e->wf[f].p, 0, sizeof(float) * e->n, e->st));
+static void zero_wavefields(Engine* e, int fields) {
+    for (int f = 0; f < fields; f++) EIO_CUDA(cudaMemsetAsync(e->wf[f].p, 0, sizeof(float) * e->n, e->st));
 }
 
 static void check_launch() {
@@ -1360,11 +1359,10 @@ struct Resident {
     int nb;
     ResPlan p;
     std::vector<ResPoints> inj, ext;
-    std::vector<ResShot> sh;
-    std::vector<ResStep> steps;
+    std::vector<char> host;     // the tables on their way to the device
     int inj_cap = 0, ext_cap = 0;
 
-    Resident(Engine* const* engines, int n) : es(engines), nb(n), inj(n), ext(n), sh(n) {}
+    Resident(Engine* const* engines, int n) : es(engines), nb(n), inj(n), ext(n) {}
 
     // within the resident loop's sizes, and free to take it
     bool small(int adj) const {
@@ -1407,28 +1405,44 @@ struct Resident {
         return false;
     }
 
+    // The tables of a call, one block on the device: steps, shots, then per shot the source map and the first
+    // point of each CTA and the points of sources (k = 0) and receivers.
+    struct Tab {
+        size_t map = 0, first[2] = {0, 0}, pt[2] = {0, 0};
+    };
+    std::vector<Tab> tab;
+    size_t tab_shot = 0, tab_bytes = 0;
+    const ResPoints& points(int i, int k) const { return k ? ext[i] : inj[i]; }
+
     // The plan's device buffers (the edge slots are some MB).  False where they do not fit: the step launches,
     // which need none of them, may still.
     bool reserve() {
         Engine* e0 = es[0];
+        size_t at = 0;
+        auto take = [&](size_t bytes) {
+            const size_t was = at;
+            at += (bytes + 15) / 16 * 16;
+            return was;
+        };
+        take(sizeof(ResStep) * (size_t)(e0->nts - 1) * e0->S);
+        tab_shot = take(sizeof(ResShot) * nb);
+        tab.resize(nb);
+        for (int i = 0; i < nb; i++)
+            for (int k = 0; k < 2; k++) {
+                const ResPoints& r = points(i, k);
+                if (!r.any) continue;
+                if (k == 0) tab[i].map = take(sizeof(short) * r.map.size());
+                tab[i].first[k] = take(sizeof(int) * r.first.size());
+                tab[i].pt[k] = take(sizeof(ResPoint) * r.pt.size());
+            }
+        tab_bytes = at;
         try {
             e0->res_x.ensure(sizeof(uint4) * slots() * nb);
-            e0->res_shot.ensure(sizeof(ResShot) * nb);
-            e0->res_step.ensure(sizeof(ResStep) * (size_t)(e0->nts - 1) * e0->S);
-            for (int i = 0; i < nb; i++)
-                for (int k = 0; k < 2; k++) {
-                    const ResPoints& r = k ? ext[i] : inj[i];
-                    if (!r.any) continue;
-                    if (k == 0) es[i]->res_map.ensure(sizeof(short) * r.map.size());
-                    es[i]->res_first[k].ensure(sizeof(int) * r.first.size());
-                    es[i]->res_pt[k].ensure(sizeof(ResPoint) * r.pt.size());
-                }
+            e0->res_tab.ensure(tab_bytes);
         } catch (const Error& x) {
             if (x.code != EIO_ERR_NOMEM) throw;
-            for (int i = 0; i < nb; i++)
-                for (DBuf* b : {&es[i]->res_x, &es[i]->res_shot, &es[i]->res_step, &es[i]->res_map, &es[i]->res_first[0],
-                                &es[i]->res_first[1], &es[i]->res_pt[0], &es[i]->res_pt[1]})
-                    b->release();
+            e0->res_x.release();
+            e0->res_tab.release();
             return false;
         }
         return true;
@@ -1437,72 +1451,67 @@ struct Resident {
     // edge slots of one shot, in uint4
     size_t slots() const { return (size_t)4 * 2 * res_edge(p.mq, p.mx) * p.ctas(); }
 
-    // tables of every shot on its engine's stream (its signal buffers are set up);
-    // the first engine's stream is to wait for the others before run()
-    void prepare() {
-        Engine* e0 = es[0];
-        for (int i = 0; i < nb; i++) {
-            Engine* e = es[i];
-            ResShot& s = sh[i];
-            memset(&s, 0, sizeof(s));
-            for (int f = 0; f < 5; f++) {
-                s.lev[0][f] = e->wf[f].f();
-                s.lev[1][f] = e->wf[5 + f].f();
-                s.par[f] = mpar(e0, f) + (long long)e->win_ix0 * e->nz;
-                s.inj_sig[f] = e->sig_in[f].f(); s.inj_ld[f] = inj[i].ld[f];
-                s.ext_sig[f] = e->sig_out[f].f(); s.ext_ld[f] = ext[i].ld[f];
-            }
-            s.dampz = e->dampz.f();
-            s.dampx = e->windowed ? e->dampx_w.f() : e->dampx.f();
-            s.nz = e->nz; s.nx = e->nx; s.Pz = p.Pz; s.Px = p.Px;
-            s.xbuf = static_cast<uint4*>(e0->res_x.p) + slots() * i;
-            for (int k = 0; k < 2; k++) {
-                const ResPoints& r = k ? ext[i] : inj[i];
-                if (!r.any) continue;
-                if (k == 0) upload(e->res_map, r.map.data(), sizeof(short) * r.map.size(), e->st);
-                upload(e->res_first[k], r.first.data(), sizeof(int) * r.first.size(), e->st);
-                upload(e->res_pt[k], r.pt.data(), sizeof(ResPoint) * r.pt.size(), e->st);
-            }
-            if (inj[i].any) {
-                s.inj_map = static_cast<const short*>(e->res_map.p);
-                s.inj_first = static_cast<const int*>(e->res_first[0].p);
-                s.inj_pt = static_cast<const ResPoint*>(e->res_pt[0].p);
-            }
-            if (ext[i].any) {
-                s.ext_first = static_cast<const int*>(e->res_first[1].p);
-                s.ext_pt = static_cast<const ResPoint*>(e->res_pt[1].p);
-            }
-        }
-    }
-
-    // every fine step, on the first engine's stream.  The adjoint's wavefield
-    // levels must be zero; this object's tables are read until the stream is done.
+    // Every fine step, on the first engine's stream, which waits for the others' signal buffers.  The adjoint's
+    // wavefield levels must be zero; the host tables are read until the stream is done.
     void run(int adj) {
         Engine* e = es[0];
         const float* F = e->filt.data();
-        const int h = e->h, S = e->S;
-        steps.clear();
-        steps.reserve((size_t)(e->nts - 1) * S);
-        for (int k = 0; k < (e->nts - 1) * S; k++) {
+        const int h = e->h, S = e->S, nsteps = (e->nts - 1) * S;
+        host.resize(tab_bytes);
+        ResStep* const steps = reinterpret_cast<ResStep*>(host.data());
+        for (int k = 0; k < nsteps; k++) {
             // engine_nl's order and weights
             const int its = adj ? e->nts - 2 - k / S : k / S, it2 = adj ? S - 1 - k % S : k % S + 1;
             const int ki = adj ? it2 + 1 : it2 - 1;
-            ResStep r;
+            ResStep& r = steps[k];
             r.inj_t = its; r.iw0 = F[ki]; r.iw1 = F[h + ki];
             r.ext_t = its; r.ew0 = F[it2]; r.ew1 = F[h + it2];
             r.ext_op = k == 0 ? RES_LOAD : k % S ? 0 : adj ? RES_DOWN : RES_UP;
             r.pad = 0;
-            steps.push_back(r);
         }
-        steps.back().ext_op |= RES_STORE;
-        upload(e->res_shot, sh.data(), sizeof(ResShot) * nb, e->st);
-        upload(e->res_step, steps.data(), sizeof(ResStep) * steps.size(), e->st);
+        steps[nsteps - 1].ext_op |= RES_STORE;
+        const char* const dev = static_cast<const char*>(e->res_tab.p);
+        auto put = [&](size_t at, const void* p, size_t bytes) { memcpy(host.data() + at, p, bytes); };
+        for (int i = 0; i < nb; i++) {
+            const Engine* ei = es[i];
+            ResShot s;
+            memset(&s, 0, sizeof(s));
+            for (int f = 0; f < 5; f++) {
+                s.lev[0][f] = ei->wf[f].f();
+                s.lev[1][f] = ei->wf[5 + f].f();
+                s.par[f] = mpar(e, f) + (long long)ei->win_ix0 * ei->nz;
+                s.inj_sig[f] = ei->sig_in[f].f(); s.inj_ld[f] = inj[i].ld[f];
+                s.ext_sig[f] = ei->sig_out[f].f(); s.ext_ld[f] = ext[i].ld[f];
+            }
+            s.dampz = ei->dampz.f();
+            s.dampx = ei->windowed ? ei->dampx_w.f() : ei->dampx.f();
+            s.nz = ei->nz; s.nx = ei->nx; s.Pz = p.Pz; s.Px = p.Px;
+            s.xbuf = static_cast<uint4*>(e->res_x.p) + slots() * i;
+            for (int k = 0; k < 2; k++) {
+                const ResPoints& r = points(i, k);
+                if (!r.any) continue;
+                put(tab[i].first[k], r.first.data(), sizeof(int) * r.first.size());
+                put(tab[i].pt[k], r.pt.data(), sizeof(ResPoint) * r.pt.size());
+            }
+            if (inj[i].any) {
+                put(tab[i].map, inj[i].map.data(), sizeof(short) * inj[i].map.size());
+                s.inj_map = reinterpret_cast<const short*>(dev + tab[i].map);
+                s.inj_first = reinterpret_cast<const int*>(dev + tab[i].first[0]);
+                s.inj_pt = reinterpret_cast<const ResPoint*>(dev + tab[i].pt[0]);
+            }
+            if (ext[i].any) {
+                s.ext_first = reinterpret_cast<const int*>(dev + tab[i].first[1]);
+                s.ext_pt = reinterpret_cast<const ResPoint*>(dev + tab[i].pt[1]);
+            }
+            put(tab_shot + sizeof(ResShot) * i, &s, sizeof(s));
+        }
+        upload(e->res_tab, host.data(), tab_bytes, e->st);
         EIO_CUDA(cudaMemsetAsync(e->res_x.p, 0, sizeof(uint4) * slots() * nb, e->st));   // no stale step matches
         ResArgs a;
         memset(&a, 0, sizeof(a));
-        a.shot = static_cast<const ResShot*>(e->res_shot.p);
-        a.step = static_cast<const ResStep*>(e->res_step.p);
-        a.nsteps = (int)steps.size();
+        a.shot = reinterpret_cast<const ResShot*>(dev + tab_shot);
+        a.step = reinterpret_cast<const ResStep*>(dev);
+        a.nsteps = nsteps;
         a.nserv = p.serv;
         a.pub = p.pub ? 1 : 0;
         a.per_shot = p.ctas();
@@ -1535,10 +1544,9 @@ void engine_nl(Engine* e, int adj, float* const model[5], float* const data[5], 
         Resident r(&e, 1);
         if (r.plan(&g, adj)) {
             err_reset(e);
-            if (adj) zero_wavefields(e);
+            if (adj) zero_wavefields(e, 10);
             stage_in(e, adj ? data : model, r.inj[0].ld, e->nts, e->sig_in);
             zero_out(e, r.ext[0].ld, e->nts, e->sig_out);
-            r.prepare();
             r.run(adj);
             check_launch();
             stage_out(e, r.ext[0].ld, e->nts, e->sig_out, adj ? model : data);
@@ -2452,6 +2460,12 @@ void engine_nl_shots_batch(Engine* const* es, int nb, int adj, float* const* mod
             dm[f] = e->stage_a[f].f();
         }
         stage_receivers(e, adj, g[i], rec + 4 * i, adj ? dataIrreg[i] : nullptr, dr);
+        if (resident) {   // neither tile lists nor, forward, the wavefield levels
+            if (adj) zero_wavefields(e, 10);
+            stage_in(e, adj ? dr : dm, res.inj[i].ld, e->nts, e->sig_in);
+            zero_out(e, res.ext[i].ld, e->nts, e->sig_out);
+            continue;
+        }
         build_points(e, g[i].srcPos, g[i].nSrc, src[i]);
         build_points(e, g[i].recPos, g[i].nRec, recp[i]);
         StepArgs& a = b.a[i];
@@ -2474,7 +2488,6 @@ void engine_nl_shots_batch(Engine* const* es, int nb, int adj, float* const* mod
         }
         max_tiles = std::max(max_tiles, e->ntiles);
     }
-    if (resident) res.prepare();
     for (int i = 1; i < nb; i++) {
         EIO_CUDA(cudaEventRecord(es[i]->ev_sync, es[i]->st));
         EIO_CUDA(cudaStreamWaitEvent(e0->st, es[i]->ev_sync, 0));
@@ -2521,12 +2534,12 @@ void engine_nl_shots_batch(Engine* const* es, int nb, int adj, float* const* mod
         if (!adj) {
             float* dr[5];
             for (int f = 0; f < 5; f++) dr[f] = e->stage_b[f].f();
-            stage_out(e, recp[i].ld, e->nts, e->sig_out, dr);
+            stage_out(e, resident ? res.ext[i].ld : recp[i].ld, e->nts, e->sig_out, dr);
             return_receivers(e, rec + 4 * i, dataIrreg[i]);
         } else {
             float* dm[5];
             for (int f = 0; f < 5; f++) dm[f] = e->stage_a[f].f();
-            stage_out(e, src[i].ld, e->nts, e->sig_out, dm);
+            stage_out(e, resident ? res.ext[i].ld : src[i].ld, e->nts, e->sig_out, dm);
             for (int f = 0; f < 5; f++)
                 d2h(e, modelReg[5 * i + f], e->stage_a[f], (size_t)g[i].nSrc[kFieldGrid[f]] * e->nts);
         }
