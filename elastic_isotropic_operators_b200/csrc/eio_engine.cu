@@ -1556,7 +1556,7 @@ void engine_nl(Engine* e, int adj, float* const model[5], float* const data[5], 
             return;
         }
     }
-    choose_kernel(e, small && way);   // it serves the Born operators too: timed without the free surface
+    if (!e->fs) choose_kernel(e, small && way);   // the free surface has one kernel
     FsScope fs_scope(e);
     err_reset(e);
     PointList src, rec;

@@ -1299,7 +1299,7 @@ static int nl_forward_impl(eio_ctx* c, int add, int nExp, int nModelExp, const f
             nl_forward_batched(c, add, nExp, nModelExp, model, data, src, rec, nRecGeom, dslice, mslice);
             return;
         }
-        const int nl = ensure_lanes(c, nExp, false, true);
+        const int nl = ensure_lanes(c, nExp, false, !c->fd.p.surfaceCondition);
         std::vector<float*> tmp(nl);
         for (int k = 0; k < nl; k++) tmp[k] = add ? lane_staging(c, k, dslice) : nullptr;
         run_lanes(c, nl, nExp, [&](int k, Engine* eng, int e) {
@@ -1364,7 +1364,7 @@ static int nl_adjoint_impl(eio_ctx* c, int add, int nExp, int nModelExp, float* 
             nl_adjoint_batched(c, nExp, nModelExp, model, data, src, rec, nRecGeom, dslice, mslice);
             return;
         }
-        const int nl = ensure_lanes(c, nExp, false, true);
+        const int nl = ensure_lanes(c, nExp, false, !c->fd.p.surfaceCondition);
         // constant source signal: every shot stacks into one model (nonlinearPropElasticShotsGpu.cpp:384-417),
         // here one partial stack per lane, added in lane order
         std::vector<std::vector<float>> slice(nl, std::vector<float>(mslice, 0.f));

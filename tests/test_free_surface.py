@@ -113,16 +113,24 @@ def test_reference_free_surface_adjoint_is_not_an_adjoint():
     assert errs[0] < 1e-12 and errs[1] > 1e-1
 
 
-def test_kernel_choice_ignores_the_free_surface():
-    """A context's step kernel is timed without the free surface, which has one kernel only: with it every
-    candidate ran that kernel and chance picked one, mostly a sweep, for the Born calls that follow.  On this
-    grid the sweep is never the fastest."""
-    w = synthetic.small(nz=600, nx=1000, nts=3, nshots=1, surface=1)
+@pytest.mark.parametrize("shots", [1, 3])
+def test_free_surface_calls_time_no_kernel(shots):
+    """The free surface has one kernel.  The candidates of the Born operators, timed with it switched on, were
+    all that kernel and chance picked one, mostly a sweep; on this grid the sweep is never the fastest."""
+    w = synthetic.small(nz=600, nx=1000, nts=3, nshots=shots, surface=1)
     src, rec = w.geometry()
     op = prop.nonlinearPropElasticShotsGpu(w.elastic, w.par, *src, *rec)
     m, d = op.modelSpace(), op.dataSpace()
     m.getNdArray()[...] = w.source_signal()[None]
+
+    def kernel():
+        v = [ctypes.c_int() for _ in range(4)]
+        _lib.check(op._L.eio_ctx_get_kernel(op.ctx, *[ctypes.byref(x) for x in v]))
+        return tuple(x.value for x in v)
+
+    before = kernel()
     op.forward(False, m, d)
-    kind = ctypes.c_int()
-    _lib.check(op._L.eio_ctx_get_kernel(op.ctx, ctypes.byref(kind), None, None, None))
-    assert kind.value != 1
+    op.adjoint(False, m, d)
+    assert kernel() == before
+    _lib.check(op._L.eio_ctx_autotune(op.ctx, None, None, None, None))
+    assert kernel()[0] != 1
