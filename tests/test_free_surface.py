@@ -134,3 +134,41 @@ def test_free_surface_calls_time_no_kernel(shots):
     assert kernel() == before
     _lib.check(op._L.eio_ctx_autotune(op.ctx, None, None, None, None))
     assert kernel()[0] != 1
+
+
+@pytest.mark.parametrize("nz,nx,nts", [(136, 88, 60), (200, 136, 60), (216, 72, 41)])
+def test_free_surface_over_several_tiles_vs_oracle(nz, nx, nts):
+    """Two to four tiles along z (64 rows each, the last one ragged): the top pass belongs to the first."""
+    w = synthetic.small(nz=nz, nx=nx, nts=nts, surface=1, nrec=10)
+    r = reg_inputs(w, "f", seed=5)
+    c = Ctx(w)
+    try:
+        for adj in (0, 1):
+            m, d = [x.copy() for x in r["model"]], [x.copy() for x in r["data"]]
+            r["orc"].nl_prop(adj, r["g"], r["med"], m, d, r["sp"], r["rp"])
+            pm, pd = c.nl(adj, r["model"], r["data"], r["sp"], r["rp"])
+            got, want = (pm, m) if adj else (pd, d)
+            assert rel(got, want) < TOL32, (adj, rel(got, want))
+    finally:
+        c.close()
+
+
+@pytest.mark.parametrize("nz", [72, 136])
+def test_free_surface_saved_wavefield_vs_oracle(nz):
+    """The saved levels are those before the next step's top pass, all rows of them."""
+    w = synthetic.small(nz=nz, nts=60, surface=1)
+    w.par.set("saveWavefield", "1")
+    w.par.set("wavefieldShotNumber", "1")
+    src, rec = w.geometry()
+    op = prop.nonlinearPropElasticShotsGpu(w.elastic, w.par, *src, *rec)
+    m, d = op.modelSpace(), op.dataSpace()
+    m.getNdArray()[...] = w.source_signal()[None]
+    op.forwardWavefield(False, m, d)
+    want, wantW = O.nl_forward(O.Oracle("f"), O.Case.from_workload(w), m.getNdArray(), wshot=1)
+    W = op.getWavefield().getNdArray()
+    assert O.rel_l2(d.getNdArray(), want) < TOL32
+    for f in range(5):
+        assert np.abs(wantW[:, f]).max() > 0
+        assert O.rel_l2(W[:, f], wantW[:, f]) < TOL32, f
+        top = slice(4, 14)                 # the surface, the rows above it and the rows it mirrors
+        assert O.rel_l2(W[:, f, :, top], wantW[:, f, :, top]) < TOL32, f

@@ -295,3 +295,31 @@ def test_resident_without_memory_for_its_slots_takes_the_step_launches():
     finally:
         _lib.check(L.eio_set_device_memory_cap(0))
     assert _resident(op, lambda: _run(op, w))
+
+
+@pytest.mark.parametrize("nz,nx,shots,fwd,adj", [
+    # one column a unit: both directions (the adjoint's last size along z)
+    (40, 56, 1, True, True), (104, 72, 5, True, True), (312, 520, 1, True, True), (1256, 56, 2, True, True),
+    (136, 264, 5, True, True), (2504, 72, 1, True, True),
+    # two columns a unit, one and two rounds: the forward only
+    (312, 600, 1, True, False), (216, 440, 2, True, False), (600, 72, 6, True, False), (72, 344, 8, True, False),
+    (408, 1016, 1, True, False), (600, 696, 1, True, False),
+    # just above the size rule
+    (408, 1032, 1, False, False)])
+def test_resident_route_and_bits(nz, nx, shots, fwd, adj):
+    """Each direction takes the resident loop where the size rule says so, and gives the step launches' bits."""
+    # more fine steps than the shots' other launches, which is what the counters tell apart
+    w = synthetic.small(nz=nz, nx=nx, nts=12 + 20 * shots, nshots=shots, nrec=min(20, (nx - 40) // 2), seed=nz + nx)
+    op, pinned = _pair(w)
+    for name, resident in (("forward", fwd), ("adjoint", adj)):
+        out = []
+        for o in (op, pinned):
+            m, d = o.modelSpace(), o.dataSpace()
+            m.getNdArray()[...] = w.source_signal()[None]
+            d.getNdArray()[...] = np.random.default_rng(3).standard_normal(d.getNdArray().shape).astype(np.float32)
+            call = lambda: getattr(o, name)(False, m, d)     # noqa: B023,E731
+            call()                                           # a first call may time kernels
+            assert _resident(o, call) == (resident and o is op), name
+            out.append((d if name == "forward" else m).getNdArray().copy())
+        assert np.abs(out[1]).max() > 0
+        np.testing.assert_array_equal(*out)
