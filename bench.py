@@ -529,11 +529,11 @@ def run_reference(args, ws, rank, local):
                 "Born drivers index the history with the 32-bit product its*nz*nx (kernelsGpuElastic.cu:1342), "
                 "which overflows here (5000*1000*3400 >= 2^31)"}
     w = synthetic.born_600x1800(nts=args.nts, nshots=1, seed=2024)
-    if not O.RefGpu.available("f"):
-        return run_reference_port(args, w, "oracle/_ref not built (reference tree absent at build time)")
     import torch
     if not torch.cuda.is_available():
         return run_reference_port(args, w, "no CUDA device on this machine")
+    if not O.RefGpu.available("f"):
+        return run_reference_port(args, w, "oracle/_ref not built (reference tree absent at build time)")
     sample_note = ""
     if not O.RefGpu.born_supported(O.Case.from_workload(w).grid()):
         # The reference's Born drivers index their Vx/Vz history with the 32-bit product
