@@ -1162,7 +1162,7 @@ static void err_reset(Engine* e) {
 static void err_check(Engine* e) {
     int flag = 0;
     EIO_CUDA(cudaMemcpy(&flag, e->err.p, sizeof(int), cudaMemcpyDeviceToHost));
-    if (flag) throw Error(EIO_ERR_TIMEOUT, "a TMA pipeline wait timed out in the step kernel (output incomplete)");
+    if (flag) throw Error(EIO_ERR_TIMEOUT, "a device wait timed out: a step kernel's copies or a neighbour of the time loop (output incomplete)");
 }
 
 void engine_set_wait_limit(Engine* e, long long polls) { e->wait_limit = polls < 0 ? WAIT_LIMIT : polls; }
@@ -1211,19 +1211,22 @@ struct ResPlan {
 // dynamic shared memory of a CTA: the 227 KB it can have less the kernel's static part
 constexpr size_t RES_SMEM = 232448 - 1024;
 // Cells of a launch (all its shots) up to which the resident loop is taken,
-// forward and adjoint (which moves the fields themselves through L2).  It is
-// bound by the exchange of edges, a per-step launch by its latency on small
-// grids and by shared memory on large ones.  Microseconds a fine step, resident
-// against k_step: 312 x 520 (162 k cells) 4.2 / 6.1 forward, 4.5 / 6.2 adjoint;
-// three shots of 312 x 424 (397 k) 6.3 / 12.2 forward, 11.7 / 11.5 adjoint;
-// 1000 x 536 (536 k) 10.3 / 11.0 forward.
+// forward and adjoint (which moves the fields themselves through L2 and asks
+// for one column a unit besides, Resident::plan).  The loop is bound by the
+// exchange of edges, a per-step launch by its latency on small grids and by
+// shared memory on large ones.  Call time over the step launches', 65 sizes of
+// one to eight shots, 150 samples: forward 0.60 to 0.98 up to 418 k cells (0.73
+// at 485 k and 0.80 at 542 k, so the line lies short of where they meet);
+// adjoint with one column 0.66 to 0.97, up to 180 k cells.
 constexpr long long RES_CELLS[2] = {420000, 200000};
 
 // Every way to cut an nz x nx grid (smallest window nx_min) into at most `ctas`
 // rectangles that the kernel can run, cheapest first.  The cost model: a unit
 // of the largest rectangle takes its LDS/STS.128 (51 a column, 37 for each of
 // two: an eighth of a cycle per lane) and the issue of its 410 instructions a
-// column; a phase cannot be shorter than the exchange of edges.
+// column; a phase cannot be shorter than the exchange of edges.  Its constants
+// only have to order the plans: at eight sizes of one to five shots the first
+// plan was within 6 % of the best of the first eight, at 72 x 104 16 % behind it.
 static std::vector<ResPlan> res_plans(int nz, int nx, int nx_min, int ctas) {
     std::vector<ResPlan> out;
     const int nq = (nz - 2 * FAT) / 4, nc = nx - 2 * FAT, nc_min = nx_min - 2 * FAT;

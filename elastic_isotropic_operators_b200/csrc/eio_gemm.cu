@@ -1303,8 +1303,9 @@ __global__ void __launch_bounds__(T_THREADS) k_conv_halo(const __grid_constant__
 // ---------------------------------------------------------------------------
 // k_wgrad_halo: the weight gradients of wide images with the same halo stages.
 // k_conv_tma fetches the nine shifted copies of x, and dz once per 128 rows of
-// the result: 12 box rows a pixel at 32 channels (27 at 96).  Here a stage is R image rows of x with their halo ((R + 2) x 136 pixels
-// per channel block) and R x 128 pixels of dz: 3 box rows a pixel.  The product
+// the result: 12 box rows a pixel at 32 channels (27 at 96).  Here a stage is R
+// image rows of x with their halo ((R + 2) x 136 pixels per channel block) and R x
+// 128 pixels of dz: 3 box rows a pixel.  The product
 // of column offset dx is one MN-major operand whose blocks of cb channels are the
 // image rows below each other (block stride one row of the slab): 128 / cb
 // vertical taps at once, those past the third computed and left out.  One
@@ -1733,6 +1734,7 @@ bool halo_plan(int n, int h, int w, int cin, int cout, HaloPlan* p)
         for (int ctas = std::min(4, 512 / talloc); ctas >= 1; ctas--) {
             const size_t most = H_SM / ctas - 2048;     // less the static part and the reserve
             const long long st = ((long long)most - 1024 - (long long)wts) / (long long)stage;
+            // a third and fourth CTA only with three stages each; with two 0.80 to 1.12 of the time
             if (st < 2 || (st < 3 && ctas > 2)) continue;
             p->r = r;
             p->ctas = ctas;
@@ -1830,6 +1832,7 @@ bool wgrad_plan(int n, int h, int w, int cin, int cout, WgradPlan* p)
         for (int ctas = std::min(4, 512 / talloc); ctas >= 1; ctas--) {
             const size_t most = H_SM / ctas - 2048;
             const long long st = ((long long)most - 1024 - (long long)tail) / (long long)stage;
+            // as halo_plan
             if (st < 2 || (st < 3 && ctas > 2)) continue;
             // A CTA's one partial result pays off over several tiles; k_conv_tma splits small images finer.
             // Time over k_conv_tma's: two or more CTAs per SM 0.93 to 1.04 at 3.5 rows of 128 pixels an SM, 0.62

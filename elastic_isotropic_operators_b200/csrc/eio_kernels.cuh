@@ -624,7 +624,7 @@ __device__ __forceinline__ void step_tail(const StepArgs& a, float* scratch, int
 // store: every tile of the top row applies it to its staged copy of the current
 // level (fs_top_staged) and to the old level as it loads it (fs_top_old), which
 // is the current level the step before applied it to.  A launch of its own
-// before each step broke the overlap of the step launches: 12.9 -> 6.4 us a
+// before each step broke the overlap of the step launches: 13.6 -> 7.9 us a
 // step on 328 x 520.
 __device__ __forceinline__ void fs_top_staged(float* sm, int tid)
 {

@@ -3,14 +3,14 @@
 // adjoint: the products its stencils read) held in shared memory throughout.
 //
 // Bound of the per-step launches on small grids: latency.  A step of k_step
-// takes 6 us at 312 x 520 and 7 us at 72 x 104, whatever its size: launch,
+// takes 6.5 us at 312 x 520 and 5.2 at 72 x 104, whatever its size: launch,
 // loads, barrier, stencils, tail, one after the other in one wave.  Here a CTA
 // owns a rectangle of the grid (one CTA per SM, the rectangles tile the grid)
-// and only the edges of the rectangles travel.  Measured (B200, per fine step):
-// 72 x 104 6.8 -> 2.9 us, 312 x 520 6.1 -> 4.2 us (adjoint 6.2 -> 4.5), three
-// shots of 312 x 424 12.2 -> 6.3 us; what is left is the exchange of edges,
-// more than 1 us a phase from store to arrival.  At 1000 x 536 the two meet
-// (10.3 against 11 us), so larger grids keep their launches.
+// and only the edges of the rectangles travel.  Measured (B200, a fine step, from
+// calls of two record lengths): 72 x 104 5.2 -> 2.65 us (adjoint 5.6 -> 2.8), 312 x
+// 520 6.5 -> 4.0 (6.75 -> 4.3), three shots of 312 x 424 8.8 -> 6.4, 408 x 1016 8.5
+// -> 6.0; what is left is the exchange of edges, about 1 us a phase from store to
+// arrival (at 312 x 520 L2 moves 9 % of what it can, shared memory 49 %).
 //
 // Leapfrog in two phases.  n = d (d o + D(c)) updates the velocities from the
 // stresses and the stresses from the velocities, so a step is two independent
@@ -109,8 +109,9 @@ constexpr size_t res_smem(int mq, int mx, int inj_cap, int ext_cap) {
     return sizeof(float) * ((size_t)10 * res_field(mq, mx) + 4 * mq + (mx + 3) / 4 * 4 + 4 * res_edge(mq, mx) +
                             (inj_cap ? res_rows(mq) * mx / 2 : 0) + (size_t)RES_INJ * inj_cap + (size_t)RES_EXT * ext_cap);
 }
-// Most threads of a CTA: 128 registers each.  At 768 (80 registers) the phases spilt 200 to 600 bytes a
-// thread and a step of 312 x 520 took 6.7 us (adjoint 7.4) instead of 4.2 (4.5).
+// Most threads of a CTA: 128 registers each, of which the phases spill 8 bytes a thread (adjoint 12, two columns
+// 48).  At 768 (80 registers) they spilt 200 to 600 and a step of 312 x 520 took 6.7 us (adjoint 7.4) instead of
+// 4.0 (4.3).
 constexpr int RES_THREADS = 512;
 
 __device__ __forceinline__ void ll_store(uint4* p, float4 v, unsigned tag)

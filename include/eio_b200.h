@@ -185,7 +185,8 @@ int eio_ctx_set_kernel(eio_ctx *c, int kind, int tz, int cw, int cpr);
 int eio_ctx_get_kernel(const eio_ctx *c, int *kind, int *tz, int *cw, int *cpr);
 int eio_ctx_autotune(eio_ctx *c, int *kind, int *tz, int *cw, int *cpr);
 /* Bound of the TMA-pipeline waits of the sweep (kind 1) and tile (kind 2)
- * kernels, in mbarrier try_wait polls (no reference counterpart: the
+ * kernels, in mbarrier try_wait polls, and of the small-grid time loop's waits
+ * for its neighbours' edges, in polls of a slot (no reference counterpart: the
  * reference's kernels have no device-side waits).  A wait that runs out sets
  * the context's error flag; the CTA then waits for its copies still in flight
  * (with a fixed long bound that this setting does not shorten) and returns,
@@ -518,7 +519,10 @@ int eio_gemm_status(int reset, int *err);
  * forces the copy loop everywhere; 1 runs the TMA kernel with one CTA per SM,
  * 2 with up to two (tiles up to 128 columns), 3 (default) with up to four
  * (three for 64-column tiles, four up to 32): fewer stages each, more copies
- * in flight per SM.  Process-wide. */
+ * in flight per SM.  Mode 3 also selects the kernels that fetch a tile once,
+ * with its halo, for all nine taps: widths that are multiples of 128, output
+ * channels a multiple of 16 up to 96 (weight gradient: 16, 32 or 64), and sizes
+ * where they are the faster ones.  Process-wide. */
 int eio_unet_set_tma(int on);
 int eio_unet_get_tma(int *on);
 /* 3x3 convolution (zero padding) as an implicit GEMM on tcgen05: y[p][co] =
