@@ -730,7 +730,15 @@ def run_ours_nl(args, ws, rank, local):
     t_ms = max_over_ranks(ws, t_ms)
     avg = st["avg_ms"]
     peak, pk = measured_peak()
-    ach = st["bytes_per_cell"] * cells / (avg * 1e-3) / 1e9
+    if st["launches"] < st["step_launches"]:
+        # both levels stay in shared memory: neither HBM bytes nor FLOPs bound a step, the exchange of edges does
+        roof = {"bound": "latency", "achieved": round(avg * 1e3, 3), "peak": None, "unit": "us per fine step",
+                "frac": None, "traffic": None, "kernel": "k_resident (every fine step in one launch)"}
+    else:
+        ach = st["bytes_per_cell"] * cells / (avg * 1e-3) / 1e9
+        roof = {"bound": "hbm", "achieved": round(ach, 1), "peak": peak, "unit": "GB/s",
+                "frac": round(ach / peak, 4), "traffic": None, "peak_source": pk, "kernel": kernel_name(L, ctx),
+                "avg_launch_us": round(avg * 1e3, 3), "algorithmic_bytes_per_launch": st["bytes_per_cell"] * cells}
     model = nl.modelSpace()
     model.getNdArray()[...] = w.source_signal()[None]
     data = nl.dataSpace()
@@ -758,12 +766,7 @@ def run_ours_nl(args, ws, rank, local):
             "e2e": {"value": round(ws * upd * args.steps / t_e2e / 1e9, 3), "unit": "Gcell-updates/s",
                     "h2d_bytes_per_step": int(sum(4 * a.size for a in reg)),
                     "d2h_bytes_per_step": int(sum(4 * t.numel() for t in d_dev))},
-            "roofline": {"bound": "hbm", "achieved": round(ach, 1), "peak": peak, "unit": "GB/s",
-                         "frac": round(ach / peak, 4), "traffic": None, "peak_source": pk,
-                         "kernel": "k_resident (every fine step in one launch; figures per fine step)"
-                         if st["launches"] < st["step_launches"] else kernel_name(L, ctx),
-                         "avg_launch_us": round(avg * 1e3, 3),
-                         "algorithmic_bytes_per_launch": st["bytes_per_cell"] * cells},
+            "roofline": roof,
             "cpu_baseline": cpu, "clocks": clk, "gpu_launches": st["launches"]}
 
 
@@ -1253,10 +1256,9 @@ def run_ours_cnn(args, ws, rank, local):
     if unet:
         nl = len(net.chans)
         # per conv: the forward GEMM; the ReLU adjoint (not the head), the weight-gradient GEMM and its split
-        # sum, the weight flip and the data-gradient GEMM (not the first layer); 3 poolings, 3 x (upsampling +
-        # concatenation), 3 x (concatenation adjoint + upsampling adjoint), 3 pooling adjoints; the loss and its
-        # sum; Adam per layer
-        launches_per_step = nl + (nl - 1) + 2 * nl + 2 * (nl - 1) + 3 + 6 + 6 + 3 + 2 + nl
+        # sum, the weight flip and the data-gradient GEMM (not the first layer); 3 poolings, 3 upsamplings with
+        # concatenation, their 3 adjoints, 3 pooling adjoints; the loss and its sum; Adam per layer
+        launches_per_step = nl + (nl - 1) + 2 * nl + 2 * (nl - 1) + 3 + 3 + 3 + 3 + 2 + nl
         flops, alg_bytes = unet_step_cost(net.chans, net._lvl(), batch, h, w)
     else:
         depth = len(net.chans) - 1
@@ -1279,8 +1281,8 @@ def run_ours_cnn(args, ws, rank, local):
     if unet:
         desc = ("cnn_train: %d patches of 256x256 per step, U-Net 32/64/128/256 channels (%d parameters), "
                 "2x2 average pooling, nearest upsampling, concatenated skips" % (batch, net.n_params()))
-        kern = ("k_conv_tma (tcgen05, TMA-fed implicit GEMM, up to 4 CTAs per SM) for forward, data and weight "
-                "gradients")
+        kern = ("k_conv_halo, k_wgrad_halo and k_conv_tma (tcgen05, TMA-fed implicit GEMMs) for forward, data and "
+                "weight gradients")
     else:
         desc = "cnn_train: %d patches of 256x256 per step, 6 conv layers 16-32-32-32-32-32-16" % batch
         kern = (("k_conv3_tc (tcgen05, TMEM accumulator)" if path.value == 1 else
